@@ -17,10 +17,12 @@
 // 6.8 / 7.2 / 11.4 us (11.0 / 11.5 / 11.9); experts of 128 x (768, 2048), top-8, with combine, at 1 / 4 / 8 / 12 rows 24 / 60 / 93 / 140 us
 // (with plan and dispatch on tcgen05: 48 / 91 / 121 / 145).  Beyond that the activations' fragments, read once per 16 weight rows,
 // fill the L1 pipe and the tcgen05 kernel is the faster one.
-// E4M3 weights (128 x 128 block scales) are expanded to bf16 in registers and meet the bf16 rows: nothing is quantised, the error of the
-// rows' E4M3 form is gone (logits of the DeepSeek-V3 geometry 1.2e-2 -> 8.7e-3 off fp64), and with it two launches per product.  Against the
-// quantise + tcgen05 E4M3 pair behind a norm: 24576 x 1536 at 1 / 8 rows 11.2 / 12.3 us (18.8 / 19.6), 7168 x 16384 41.3 / 47.4 (47.3 / 47.4);
-// experts of 256 x (2048, 7168), top-8, at 1 / 4 / 8 rows 86 / 266 / 468 us (129 / 326 / 497), 4.4 TB/s where the expansion bounds it.
+// E4M3 weights (128 x 128 block scales) are expanded to f16 in registers and meet the bf16 rows as f16, exactly over the range that matters
+// (sk_rows_f16): nothing is quantised, the error of the rows' E4M3 form is gone (logits of the DeepSeek-V3 geometry 1.2e-2 -> 8.7e-3 off
+// fp64), and with it two launches per product; a NaN code makes its feature NaN, as it does in the products of larger steps.  Against the
+// quantise + tcgen05 E4M3 pair: 24576 x 1536 at 1 / 8 rows behind a norm 12.5 / 13.3 us (19.2 / 19.7), 7168 x 16384 37.7 / 43.4
+// (39.8 / 40.5, with the rows' quantisation error); experts of 256 x (2048, 7168), top-8, with combine, at 1 / 4 / 8 rows 91 / 280 / 538 us
+// (133 / 337 / 564), 4.2 TB/s where the instructions of the two conversions bound it.
 // Sums run in fp32 in a fixed order (K groups of a warp, then warps), so results do not depend on scheduling; they do depend on the
 // kernel, so the batch-invariant mode, which promises the same bits at any row count, stays on the tcgen05 kernel.
 #include "cafd_api.h"
@@ -59,16 +61,35 @@ __device__ __forceinline__ uint4 sk_ldw(const uint8_t* p) {      // weights: rea
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-// Four E4M3 values -> two bf16 pairs, exactly: sign, exponent and mantissa moved to their places make the value times 2^-120 (subnormal
-// E4M3 values become subnormal bf16 ones), and the product with 2^120 is exact.  A byte beside its replicated sign, shifted by four, has
-// every bit where it belongs: four instructions per pair, which is what bounds the E4M3 form (HBM would ask for 1.5 of an SM's 4 per clock).
-// The NaN codes come out as +-480.
+// Four E4M3 codes -> two f16 pairs, exactly; the NaN codes become NaN.  (bf16 pairs, from shifts and a product with 2^120, cost four
+// instructions a pair, as much as this and the rows' conversion together, and turn the NaN codes into +-480; finding the codes beside
+// that cost a fifth more.  The experts above took 88 / 265 / 511 us without NaN, 320 / 625 us at 4 / 8 rows with it.)
 __device__ __forceinline__ void sk_expand(uint32_t v, uint32_t& lo, uint32_t& hi) {
-  uint32_t a, b;
-  asm("prmt.b32 %0, %1, %1, 0x9180;" : "=r"(a) : "r"(v));
-  asm("prmt.b32 %0, %1, %1, 0xb3a2;" : "=r"(b) : "r"(v));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(lo) : "r"((a << 4) & 0x87f087f0u), "r"(0x7b807b80u));
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(hi) : "r"((b << 4) & 0x87f087f0u), "r"(0x7b807b80u));
+  asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %2;\ncvt.rn.f16x2.e4m3x2 %0, l;\ncvt.rn.f16x2.e4m3x2 %1, h;\n}" : "=r"(lo), "=r"(hi) : "r"(v));
+}
+// A lane's 32 of the 128 bf16 values of a row that meet an E4M3 block, to f16: times the power of two that brings the largest of the 128
+// into [2^14, 2^15), so that everything down to 2^-29 of it keeps all its bits and what is smaller is off by 2^-40 of it at most, less than
+// what sums in fp32 lose.  Infinities and NaN stay.  Returns the inverse power.  Lanes 4 g ... 4 g + 3 hold the row.
+__device__ __forceinline__ float sk_rows_f16(uint32_t (&x)[16]) {
+  uint32_t m[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(m[i]) : "r"(x[i]), "r"(x[i + 8]));
+#pragma unroll
+  for (int d = 4; d; d >>= 1)
+#pragma unroll
+    for (int i = 0; i < d; ++i) asm("max.xorsign.abs.bf16x2 %0, %0, %1;" : "+r"(m[i]) : "r"(m[i + d]));
+  uint32_t top = max((m[0] >> 16) & 0x7fffu, m[0] & 0x7fffu);
+  top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+  top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+  const uint32_t e = max(top >> 7, 15u);                       // its exponent field
+  const uint32_t s = (268u - e) << 7, s2 = s | s << 16;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    uint32_t t;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(x[i]), "r"(s2));
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(x[i]) : "f"(__uint_as_float(t & 0xffff0000u)), "f"(__uint_as_float(t << 16)));
+  }
+  return __uint_as_float((e - 14u) << 23);
 }
 __device__ __forceinline__ uint4 sk_ldx(const __nv_bfloat16* p) {      // activations: shared by the SM's blocks through L1
   uint4 v;
@@ -77,6 +98,12 @@ __device__ __forceinline__ uint4 sk_ldx(const __nv_bfloat16* p) {      // activa
 }
 __device__ __forceinline__ void sk_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void sk_mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -243,27 +270,31 @@ __global__ void __launch_bounds__(kSkThreads, skinny_per_sm(kNT, kGB, kF8)) skin
               const __nv_bfloat16* xg = xr[nt] + grp * kElems;
               if constexpr (kF8) {
                 // a block's products are summed apart and scaled once
-                uint4 bx[2][2];
+                uint32_t xb[16];
 #pragma unroll
-                for (int h = 0; h < 2; ++h) { bx[h][0] = sk_ldx(xg + h * 64); bx[h][1] = sk_ldx(xg + h * 64 + 8); }
+                for (int h = 0; h < 4; ++h) {
+                  const uint4 v = sk_ldx(xg + (h >> 1) * 64 + (h & 1) * 8);
+                  xb[4 * h] = v.x; xb[4 * h + 1] = v.y; xb[4 * h + 2] = v.z; xb[4 * h + 3] = v.w;
+                }
+                const float inv = sk_rows_f16(xb);
+                const float i0 = __shfl_sync(0xffffffffu, inv, 8 * q), i1 = __shfl_sync(0xffffffffu, inv, 8 * q + 4);     // rows 2 q, 2 q + 1
                 float raw[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                   const uint32_t w0[4] = {a[i][0][h].x, a[i][0][h].y, a[i][0][h].z, a[i][0][h].w};
                   const uint32_t w1[4] = {a[i][1][h].x, a[i][1][h].y, a[i][1][h].z, a[i][1][h].w};
-                  const uint32_t xb[8] = {bx[h][0].x, bx[h][0].y, bx[h][0].z, bx[h][0].w, bx[h][1].x, bx[h][1].y, bx[h][1].z, bx[h][1].w};
 #pragma unroll
                   for (int e = 0; e < 4; ++e) {
                     uint32_t a0, a1, a2, a3;
                     sk_expand(w0[e], a0, a2);
                     sk_expand(w1[e], a1, a3);
-                    sk_mma(raw, a0, a1, a2, a3, xb[2 * e], xb[2 * e + 1]);
+                    sk_mma_f16(raw, a0, a1, a2, a3, xb[8 * h + 2 * e], xb[8 * h + 2 * e + 1]);
                   }
                 }
-                acc[nt][0] += raw[0] * sc[i][0];
-                acc[nt][1] += raw[1] * sc[i][0];
-                acc[nt][2] += raw[2] * sc[i][1];
-                acc[nt][3] += raw[3] * sc[i][1];
+                acc[nt][0] += raw[0] * i0 * sc[i][0];
+                acc[nt][1] += raw[1] * i1 * sc[i][0];
+                acc[nt][2] += raw[2] * i0 * sc[i][1];
+                acc[nt][3] += raw[3] * i1 * sc[i][1];
               } else {
                 const uint4 b0 = sk_ldx(xg), b1 = sk_ldx(xg + 32);
                 sk_mma(acc[nt], a[i][0][0].x, a[i][1][0].x, a[i][0][0].y, a[i][1][0].y, b0.x, b0.y);

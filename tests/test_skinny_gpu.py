@@ -117,3 +117,59 @@ def test_e4m3_experts_of_a_step(T, top_k, E, I, H):
         c, b = gate[ex] @ x[e // top_k].double(), up[ex] @ x[e // top_k].double()
         _close(hbuf[e], torch.nn.functional.silu(c) * b, 1.0 + c.abs() + b.abs())
         _close(out[e], down[ex] @ hbuf[e].double(), I ** 0.5 * float(hbuf[e].abs().max()))
+
+
+def test_e4m3_rows_of_any_size():
+    """Values from bf16 subnormals to near its largest number, alone in a row and side by side in one 128-wide block: off the fp64 product by
+    what fp32 sums lose (a few 2^-24 of the terms' absolute sum) and one rounding to bf16; infinities and NaN come through."""
+    from cuteafd_b200.ops import kernels as k
+    g = torch.Generator(device=DEV).manual_seed(11)
+    N, K = 256, 512
+    q, s, w = _e4m3((N, K), g)
+    x = torch.randn(8, K, device=DEV, generator=g).double()
+    x[0] *= 2.0 ** -130
+    x[1] *= 2.0 ** 112
+    x[2] *= 2.0 ** torch.randint(-60, 60, (K,), device=DEV, generator=g)
+    x[3] *= 2.0 ** torch.randint(-24, 1, (K,), device=DEV, generator=g)
+    x[4, 128:] = 0
+    x[5] = 0
+    x[6] *= 70000.0
+    x = x.to(torch.bfloat16)
+    want, size = x.double() @ w.T, x.double().abs() @ w.abs().T
+    got = k.linear_w8(x, q, s, torch.empty(8, N, dtype=torch.bfloat16, device=DEV)).double()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -20 * size + 2.0 ** -133).all()
+    x[0, 7], x[1, 300] = float("inf"), float("nan")
+    got = k.linear_w8(x, q, s, torch.empty(8, N, dtype=torch.bfloat16, device=DEV))
+    assert torch.equal(got[2:].double(), k.linear_w8(x[2:], q, s, torch.empty(6, N, dtype=torch.bfloat16, device=DEV)).double())
+    assert not got[:2].isfinite().any() and got[1].isnan().all()
+
+
+def test_e4m3_nan_codes_stay_nan():
+    """A weight row that holds one of the two NaN codes gives NaN in its feature for every row of x, zero rows included, as the tensor-core
+    products of larger steps do; every other feature is untouched."""
+    from cuteafd_b200.ops import kernels as k
+    g = torch.Generator(device=DEV).manual_seed(5)
+    T, N, K, E = 6, 256, 1152, 4
+    x = (torch.randn(T, K, device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    x[2] = 0
+    q, s, _ = _e4m3((N, K), g)
+    clean = k.linear_w8(x, q, s, torch.empty(T, N, dtype=torch.bfloat16, device=DEV))
+    bad = {0: (0, 0x7f), 5: (K - 1, 0xff), 8: (77, 0x7f), 130: (640, 0xff), N - 1: (3, 0xff)}
+    qb = q.clone()
+    for row, (col, code) in bad.items():
+        qb.view(torch.uint8)[row, col] = code
+    rows = torch.zeros(N, dtype=torch.bool, device=DEV)
+    rows[list(bad)] = True
+    for up in (None, q):
+        got = k.linear_w8(x, qb, s, torch.empty_like(clean), w_up=up, ws_up=s if up is not None else None)
+        assert got[:, rows].isnan().all() and got[:, ~rows].isfinite().all()
+        assert up is not None or torch.equal(got[:, ~rows], clean[:, ~rows])
+    assert k.linear_w8(x, q, s, torch.empty_like(clean), w_up=qb, ws_up=s)[:, rows].isnan().all()
+    (qe, se, _), (qu, su, _) = _e4m3((E, N, K), g), _e4m3((E, N, K), g)
+    qe.view(torch.uint8)[2, 9, 200] = 0x7f
+    idx = torch.tensor([[0, 1], [2, 3], [3, 0], [1, 2], [0, 3], [1, 0]], dtype=torch.int32, device=DEV)
+    h = torch.empty(T * 2, N, dtype=torch.bfloat16, device=DEV)
+    k.moe_skinny(x, 2, qe, qu, idx, h, scale=se, scale_up=su)
+    want = torch.zeros(T * 2, N, dtype=torch.bool, device=DEV)
+    want[:, 9] = idx.flatten() == 2
+    assert torch.equal(h.isnan(), want)
