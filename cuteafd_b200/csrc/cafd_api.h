@@ -80,6 +80,7 @@ typedef struct {
 } cafd_gemm_args;
 
 int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream);
+int cafd_gemm_prompt_tile(int rows, int features, int num_sms);
 
 // ---- greedy selection ----------------------------------------------------------------------------
 // out[t] = argmax over logits[t, 0:V] (row pitch ld, fp32); ties go to the lowest index and NaN is

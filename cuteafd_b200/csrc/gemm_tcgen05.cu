@@ -568,6 +568,19 @@ static int launch(const cafd_gemm_args* a, cudaStream_t stream) {
 
 }  // namespace cafd
 
+// Feature width of a dense product's 128-row tiles with tokens on the M side.  A chat-sized prompt's projection has few 128 x 256 tiles, and a
+// tile's K range is one block's serial chain: narrower tiles put more SMs to work (the sums of an element don't depend on the width), but
+// a narrow tile takes more than half a wide one's time, so they pay only while all of them run at once.  512 rows, 2048 x 4096: 32 tiles of
+// 256 50 us, 128 of 64 30 us; 777 rows: 56 of 256 47 us, 112 of 128 37 us; a router's 128 x 2048 at 777 rows 16 -> 13 us.  Where the
+// narrow ones take a second wave they lose: 640 rows, 2048 x 4096: 40 of 256 32 us, 160 of 64 49 us; 300 rows, 4096 x 14336: 48 of 256
+// 92 us, 192 of 64 160 us.
+extern "C" int cafd_gemm_prompt_tile(int rows, int features, int num_sms) {
+  const long long sms = num_sms > 0 ? num_sms : 148, m = (static_cast<long long>(rows) + 127) / 128;
+  for (int width = 64; width < 256; width *= 2)
+    if (m * ((static_cast<long long>(features) + width - 1) / width) <= sms) return width;
+  return 256;
+}
+
 extern "C" int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream_) {
   using namespace cafd;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -607,14 +620,9 @@ extern "C" int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream_) {
   }
   if (a->dual) return launch<false, true, 128, 128>(a, stream);
   if (!a->tile_expert) {
-    // A chat-sized prompt's projection has few 128 x 256 tiles, and a tile's K range is one block's serial chain: narrower tiles put more
-    // SMs to work (the sums of an element don't depend on the width).  777 rows,
-    // 2048 x 4096: 56 tiles of 256, 47 us, 112 of 128, 37 us; 512 rows 50 -> 30 us; a router's 128 x 2048 at 777 rows 16 -> 13 us.
-    const int sms = a->num_sms > 0 ? a->num_sms : 148;
-    const long long rows = (a->x_rows + 127) / 128;
-    if (rows * ((a->n_features + 255) / 256) * 4 < 3ll * sms) {
-      if (rows * ((a->n_features + 127) / 128) * 4 < 3ll * sms) return launch<false, false, 128, 64>(a, stream);
-      return launch<false, false, 128, 128>(a, stream);
+    switch (cafd_gemm_prompt_tile(a->x_rows, a->n_features, a->num_sms)) {
+      case 64: return launch<false, false, 128, 64>(a, stream);
+      case 128: return launch<false, false, 128, 128>(a, stream);
     }
   }
   return launch<false, false, 128, 256>(a, stream);

@@ -21,6 +21,21 @@ def test_projections_of_chat_sized_prompts(T, N):
         assert ((got.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * K ** 0.5).all()
 
 
+@pytest.mark.parametrize("K", [1408, 4096, 7168])
+def test_projections_do_not_depend_on_the_tile_width(K):
+    """The same rows in prompts that take tiles of 64 (up to 512 rows), 128 (777) and 256 features (2300): the same bits."""
+    from cuteafd_b200.ops import kernels as k
+    N = 2048
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, w = (torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((2300, K), (N, K)))
+    wide = k.linear(x, w, out_f32=True)
+    widths = [256]
+    for T in (129, 512, 777):
+        widths.append(k._n.cuda_lib().cafd_gemm_prompt_tile(T, N, k.num_sms()))
+        assert torch.equal(k.linear(x[:T], w, out_f32=True), wide[:T])
+    assert k._n.cuda_lib().cafd_gemm_prompt_tile(2300, N, k.num_sms()) == 256 and set(widths) == {64, 128, 256}
+
+
 @pytest.mark.parametrize("Hq,Hkv", [(32, 4), (8, 2), (5, 1)])
 @pytest.mark.parametrize("interleaved,rot,bias", [(False, 128, False), (True, 128, True), (False, 64, False), (True, 64, False)])
 def test_rope_of_a_prompt_is_that_of_its_tokens(Hq, Hkv, interleaved, rot, bias):
