@@ -1,4 +1,4 @@
-// Exact full-vocabulary target sampling on the GPU, one thread block per logit row, plus the
+// Exact full-vocabulary target sampling on the GPU, a cluster of thread blocks per logit row, plus the
 // accept-prefix scan of sample-match speculative verification.
 //
 // Filter order: allowed-token mask -> temperature -> min_p -> top_k (exactly k, lowest id wins a
@@ -10,7 +10,7 @@
 // integer, so sums are associative and the result does not depend on thread timing: the same row
 // always yields the same token.
 //
-// One cluster of eight blocks per row, each with an eighth of the vocabulary in shared memory as
+// One cluster of one to eight blocks per row, each with its share of the vocabulary in shared memory as
 // order-preserving 32-bit keys.  What bounds the kernel is the number of dependent passes, not the
 // 0.6 MB a row is read once: with one block per row, walking the row from L2 in every pass, eight
 // rows of 151936 took 371 us and 32 rows of 129280 666 us, now 32 and 44 us.  One histogram over
@@ -29,10 +29,10 @@ namespace cafd {
 namespace cg = cooperative_groups;
 
 constexpr int kSampleThreads = 512;              // at 64 registers a thread two blocks share an SM: 32 rows are one wave (1024 threads: two waves, 67 us)
-constexpr int kSampleCluster = 8;                // blocks per row (the portable cluster size)
 constexpr int kSampleBins = 256;
 constexpr int kSampleList = 2048;                // tokens that the sorted list holds
 constexpr int kSampleSmemKeys = 48 * 1024;       // keys of a slice kept in shared memory; longer slices are read again in every pass
+constexpr int kSampleKeysPair = 20 * 1024;       // up to this many two blocks share an SM
 constexpr int kLimbKeys = 1 << 17;               // slice length up to which 15-bit limbs of the masses add up in 32 bits
 constexpr float kGreedyEps = 1.0e-5f;
 
@@ -65,13 +65,10 @@ __device__ __forceinline__ float splitmix_uniform(unsigned long long seed, long 
 struct Cut { uint32_t key; int id; };     // members: key > cut.key, or key == cut.key and id <= cut.id
 
 // Histogram of one pass: a count and a mass per bin.  Masses are below 2^45: three 15-bit limbs, each with native 32-bit shared
-// atomics (a 64-bit shared add is a compare-and-swap loop).
+// atomics (a 64-bit shared add is a compare-and-swap loop); a slice too long for their sums takes two whole words.
 struct SampleHist {
   unsigned int cnt[kSampleBins];
-  union {
-    unsigned int limb[3][kSampleBins];
-    unsigned long long wide[kSampleBins];
-  };
+  unsigned int limb[3][kSampleBins];
 };
 
 struct SampleShared {
@@ -149,22 +146,27 @@ __device__ __forceinline__ void hist_clear(SampleHist& h) {
     h.limb[0][i] = 0; h.limb[1][i] = 0; h.limb[2][i] = 0;
   }
 }
-__device__ __forceinline__ void hist_add(SampleHist& h, int b, unsigned long long m, bool wide) {
-  atomicAdd(&h.cnt[b], 1u);
-  if (wide) { atomicAdd(&h.wide[b], m); return; }
+__device__ __forceinline__ void hist_add_mass(SampleHist& h, int b, unsigned long long m, bool wide) {
+  if (wide) {                                    // two words, the carry of the lower from the value it had
+    const unsigned int lo = static_cast<unsigned int>(m), was = atomicAdd(&h.limb[0][b], lo);
+    const unsigned int hi = static_cast<unsigned int>(m >> 32) + (was + lo < was ? 1u : 0u);
+    if (hi) atomicAdd(&h.limb[1][b], hi);
+    return;
+  }
   const unsigned int l0 = static_cast<unsigned int>(m) & 0x7fffu, l1 = static_cast<unsigned int>(m >> 15) & 0x7fffu, l2 = static_cast<unsigned int>(m >> 30);
   if (l0) atomicAdd(&h.limb[0][b], l0);
   if (l1) atomicAdd(&h.limb[1][b], l1);
   if (l2) atomicAdd(&h.limb[2][b], l2);
 }
 // Thread t < 256 gets bin b's count and mass over the whole cluster (after the cluster's barrier).
+template <int kC>
 __device__ __forceinline__ void hist_total(cg::cluster_group& cluster, SampleHist& h, int b, bool wide, unsigned int& c, unsigned long long& m) {
   c = 0; m = 0;
 #pragma unroll
-  for (int r = 0; r < kSampleCluster; ++r) {
+  for (int r = 0; r < kC; ++r) {
     const SampleHist* o = cluster.map_shared_rank(&h, r);
     c += o->cnt[b];
-    if (wide) m += o->wide[b];
+    if (wide) m += o->limb[0][b] + (static_cast<unsigned long long>(o->limb[1][b]) << 32);
     else m += o->limb[0][b] + (static_cast<unsigned long long>(o->limb[1][b]) << 15) + (static_cast<unsigned long long>(o->limb[2][b]) << 30);
   }
 }
@@ -172,6 +174,7 @@ __device__ __forceinline__ void hist_total(cg::cluster_group& cluster, SampleHis
 // Smallest prefix of the order, inside `cut`, whose cumulative metric reaches `target_frac` (by_mass: a fraction of the cut's total
 // mass, strict = "exceeds"; else a count).  Returns the new cut; its id is the last member of the prefix.  All threads of the cluster
 // call this with identical arguments.
+template <int kC>
 __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, Cut cut, bool by_mass, double frac, bool strict,
                              long long count_target, bool wide, SampleShared& sh) {
   const int tid = threadIdx.x, rank = static_cast<int>(cluster.block_rank());
@@ -186,13 +189,15 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
       const uint32_t key = s.key(j);
       if (!key || key < cut.key || (key == cut.key && s.id0 + j > cut.id)) continue;
       if (level > 0 && (key >> (shift + 8)) != prefix) continue;
-      hist_add(h, (key >> shift) & 255u, by_mass ? mass_of(key_value(key), s.maxp) : 0ull, wide);
+      const int b = (key >> shift) & 255u;
+      if (by_mass) hist_add_mass(h, b, mass_of(key_value(key), s.maxp), wide);
+      else atomicAdd(&h.cnt[b], 1u);
     }
     cluster.sync();
     unsigned int c = 0;
     unsigned long long m = 0;
     const int b = 255 - tid;                 // thread order = descending keys
-    if (tid < kSampleBins) hist_total(cluster, h, b, wide, c, m);
+    if (tid < kSampleBins) hist_total<kC>(cluster, h, b, wide, c, m);
     const unsigned long long v = by_mass ? m : c;
     const unsigned long long incl = block_scan(v, sh.scan);
     if (level == 0) {
@@ -226,7 +231,7 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
   cluster.sync();
   int before = 0, n_ties = 0;
 #pragma unroll
-  for (int r = 0; r < kSampleCluster; ++r) {
+  for (int r = 0; r < kC; ++r) {
     const int t = *cluster.map_shared_rank(&sh.ties, r);
     if (r < rank) before += t;
     n_ties += t;
@@ -240,7 +245,7 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
     for (int j = lo; j < hi; ++j) {
       const uint32_t key = s.key(j);
       if (key == prefix && (key > cut.key || s.id0 + j <= cut.id) && ++seen == need) {
-        for (int r = 0; r < kSampleCluster; ++r) *cluster.map_shared_rank(&sh.pick_id, r) = s.id0 + j;
+        for (int r = 0; r < kC; ++r) *cluster.map_shared_rank(&sh.pick_id, r) = s.id0 + j;
         break;
       }
     }
@@ -251,6 +256,7 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
   return out;
 }
 
+template <int kC>
 __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float* __restrict__ logits, int ld, int V, int slice,
                                                                      const SampleRow* __restrict__ rows,
                                                                      const uint32_t* __restrict__ masks,
@@ -261,7 +267,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   extern __shared__ uint32_t sm_keys[];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = static_cast<int>(cluster.block_rank());
-  const int out_row = blockIdx.x / kSampleCluster;
+  const int out_row = blockIdx.x / kC;
   const SampleRow rp = rows[out_row];
   const float* x = logits + static_cast<size_t>(rp.logits_row) * ld;
   const uint32_t* mask = rp.mask_word0 >= 0 ? masks + rp.mask_word0 : nullptr;
@@ -273,15 +279,32 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
                          !(rp.min_p >= 0.f && rp.min_p <= 1.0f) || V <= 0;
   // ---- pass A: validation, max, lowest-id argmax; the logits stay in shared memory ---------------------
   float best = -INFINITY; int bi = 0x7fffffff; int cnt = 0, bad = 0;
-#pragma unroll 8
-  for (int j = tid; j < n; j += kSampleThreads) {
-    const int i = id0 + j;
-    const float v = x[i];
-    if (in_smem) sm_keys[j] = __float_as_uint(v);
-    if (mask && !((mask[i >> 5] >> (i & 31)) & 1u)) continue;
-    ++cnt;
-    if (!isfinite(v)) { bad = 1; continue; }
-    if (v > best || (v == best && i < bi)) { best = v; bi = i; }
+  constexpr int kAhead = 8;                       // loads in flight per thread (one after the other: 256 greedy rows of 262144 604 us, now 213)
+  for (int j0 = tid; j0 < n; j0 += kAhead * kSampleThreads) {
+    float v[kAhead];
+    bool in[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      const int j = j0 + q * kSampleThreads;
+      in[q] = j < n;
+      v[q] = in[q] ? __ldcg(x + id0 + j) : 0.f;
+    }
+    if (mask) {
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int i = id0 + j0 + q * kSampleThreads;
+        if (in[q]) in[q] = (__ldcg(mask + (i >> 5)) >> (i & 31)) & 1u;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      const int j = j0 + q * kSampleThreads, i = id0 + j;
+      if (in_smem && j < n) sm_keys[j] = __float_as_uint(v[q]);
+      const bool finite = isfinite(v[q]);
+      cnt += in[q];
+      bad |= in[q] && !finite;
+      if (in[q] && finite && (v[q] > best || (v[q] == best && i < bi))) { best = v[q]; bi = i; }
+    }
   }
   for (int o = 16; o; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -305,7 +328,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   cluster.sync();
   best = -INFINITY; bi = 0x7fffffff; cnt = 0; bad = 0;
 #pragma unroll
-  for (int r = 0; r < kSampleCluster; ++r) {
+  for (int r = 0; r < kC; ++r) {
     const SampleShared* o = cluster.map_shared_rank(&sh, r);
     const float ov = o->row_v; const int oi = o->row_i;
     if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
@@ -341,7 +364,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     }
     if (!key) continue;
     const float xp = key_value(key);
-    hist_add(sh.hist[0], s.bin(xp), mass_of(xp, s.maxp), wide);
+    const int b = s.bin(xp);
+    atomicAdd(&sh.hist[0].cnt[b], 1u);
+    hist_add_mass(sh.hist[0], b, mass_of(xp, s.maxp), wide);
   }
   if (in_smem) s.keys = sm_keys;
   cluster.sync();
@@ -351,7 +376,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   const double u = static_cast<double>(uf);
   unsigned int bc = 0;
   unsigned long long bm = 0;
-  if (tid < kSampleBins) hist_total(cluster, sh.hist[0], tid, wide, bc, bm);
+  if (tid < kSampleBins) hist_total<kC>(cluster, sh.hist[0], tid, wide, bc, bm);
   const unsigned int cc = block_scan(bc, reinterpret_cast<unsigned int*>(sh.counts));
   const unsigned long long cm = block_scan(bm, sh.scan);
   if (tid == kSampleThreads - 1) { sh.acc_c = cc; sh.acc_m = cm; }
@@ -381,7 +406,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     if (rank > 0) {
       int at = 0;
 #pragma unroll
-      for (int r = 0; r < kSampleCluster; ++r)
+      for (int r = 0; r < kC; ++r)
         if (r < rank) at += *cluster.map_shared_rank(&sh.n_list, r);
       unsigned long long* dst = cluster.map_shared_rank(sh.list, 0);
       for (int j = tid; j < sh.n_list; j += kSampleThreads) dst[at + j] = sh.list[j];
@@ -438,9 +463,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   } else {
     cluster.sync();                            // every block has read the histograms that the descents reuse
     Cut cut{0u, 0x7fffffff};
-    if (use_k) cut = select_prefix(cluster, s, cut, false, 0.0, false, rp.top_k, wide, sh);
-    if (use_p) cut = select_prefix(cluster, s, cut, true, static_cast<double>(rp.top_p), false, 0, wide, sh);
-    const Cut pick = select_prefix(cluster, s, cut, true, u, true, 0, wide, sh);
+    if (use_k) cut = select_prefix<kC>(cluster, s, cut, false, 0.0, false, rp.top_k, wide, sh);
+    if (use_p) cut = select_prefix<kC>(cluster, s, cut, true, static_cast<double>(rp.top_p), false, 0, wide, sh);
+    const Cut pick = select_prefix<kC>(cluster, s, cut, true, u, true, 0, wide, sh);
     token = pick.id >= 0 ? pick.id : bi;
   }
   if (rank == 0 && tid == 0) { out_token[out_row] = token; out_status[out_row] = kSampleOk; }
@@ -464,9 +489,51 @@ __global__ void accept_prefix_kernel(const int* __restrict__ selected, const int
   bonus[s] = n > 0 ? selected[r0 + a] : -1;
 }
 
+struct SampleCall {
+  const float* logits;
+  int ld, V;
+  const SampleRow* rows;
+  const uint32_t* masks;
+  int n;
+  int *out_token, *out_status;
+};
+
+template <int kC>
+static int launch_sample(const SampleCall& c, cudaStream_t st) {
+  const int slice = c.V > 0 ? static_cast<int>((static_cast<long long>(c.V) + kC - 1) / kC) : 0;
+  const size_t smem = slice <= kSampleSmemKeys ? static_cast<size_t>(slice) * 4 : 0;
+  CAFD_CHECK_CUDA(cudaFuncSetAttribute(sample_rows_kernel<kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmemKeys * 4));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(c.n) * kC);
+  cfg.blockDim = dim3(kSampleThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = kC;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, sample_rows_kernel<kC>, c.logits, c.ld, c.V, slice, c.rows, c.masks, c.out_token,
+                                             c.out_status));
+}
+
 }  // namespace cafd
 
 using namespace cafd;
+
+// Blocks per row: eight, and fewer for a batch that would not be resident at once (two blocks to an SM) as long as a slice's keys still
+// stay in shared memory beside another block's.  Clusters of a fixed eight, and one block that reads its row again in every pass, against
+// this, us: 256 greedy rows of 8192 41 / 16 / 11, of 32000 51 / 23 / 20; 256 rows of 8192, top-k 50 and top-p 0.95, 101 / 79 / 26.  Keys
+// that don't stay in shared memory cost more than the further waves: 256 rows of 151936, top-p 0.9, 296 us with eight blocks, 555 with one.
+extern "C" int cafd_sample_cluster(int n, int V, int num_sms) {
+  int c = 8;
+  while (c > 1 && static_cast<long long>(n) * c > 2ll * num_sms && V / (c / 2) < kSampleKeysPair) c /= 2;
+  return c;
+}
 
 // rows: n 64-byte records {f32 temperature, top_p, min_p; i32 top_k; u64 seed; i64 position; i64 mask_word0;
 // i32 logits_row; 20 bytes pad}.  masks: packed allowed-token bits (bit i of word i/32), or null.
@@ -474,25 +541,17 @@ extern "C" int cafd_sample_rows(const float* logits, int ld, int V, const void* 
                                 int* out_token, int* out_status, cafd_stream_t s) {
   if (n <= 0) return 0;
   static_assert(sizeof(SampleRow) == 64, "row record is 64 bytes");
-  const int slice = (V + kSampleCluster - 1) / kSampleCluster;
-  const size_t smem = slice <= kSampleSmemKeys ? static_cast<size_t>(slice) * 4 : 0;
-  CAFD_CHECK_CUDA(cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmemKeys * 4));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(n) * kSampleCluster);
-  cfg.blockDim = dim3(kSampleThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = static_cast<cudaStream_t>(s);
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = kSampleCluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, ld, V, slice, static_cast<const SampleRow*>(rows), masks,
-                                             out_token, out_status));
+  int dev = 0, sms = 0;
+  CAFD_CHECK_CUDA(cudaGetDevice(&dev));
+  CAFD_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const SampleCall c{logits, ld, V, static_cast<const SampleRow*>(rows), masks, n, out_token, out_status};
+  cudaStream_t st = static_cast<cudaStream_t>(s);
+  switch (cafd_sample_cluster(n, V, sms)) {
+    case 8: return launch_sample<8>(c, st);
+    case 4: return launch_sample<4>(c, st);
+    case 2: return launch_sample<2>(c, st);
+  }
+  return launch_sample<1>(c, st);
 }
 
 extern "C" int cafd_accept_prefix(const int* selected, const int* draft, const int* row_start, int S, int* accepted,

@@ -96,3 +96,32 @@ def test_sample_rows_over_vocabularies(V, shape):
     st = torch.full((n,), -7, dtype=torch.int32, device=dev)
     K.sample_rows(logits.to(dev), K.pack_sample_rows(params, positions).to(dev), tok, st)
     assert st.tolist() == status and tok.tolist() == want
+
+
+@pytest.mark.parametrize("n,V,blocks", [(74, 32003, 4), (148, 32003, 2), (150, 20481, 2), (300, 1, 1), (300, 9, 1), (300, 2500, 1), (300, 20479, 1)])
+@pytest.mark.parametrize("shape", ["flat", "ties"])
+def test_sample_many_rows(n, V, blocks, shape):
+    """Batches whose rows get four, two and one block each, every third row under a mask of allowed tokens."""
+    from cuteafd_b200.ops import kernels as K
+    from cuteafd_b200.runtime.sampling import SamplingParams, select_rows
+    dev = torch.device("cuda", 0)
+    kinds = [dict(temperature=1.0), dict(temperature=0.5, top_p=0.9), dict(temperature=1.0, top_k=50, top_p=0.95), dict(temperature=2.0, top_k=3000),
+             dict(temperature=1.0, min_p=0.02, top_p=0.8), dict()]
+    params = [SamplingParams(seed=i, **kinds[i % 6]) for i in range(n)]
+    positions = [7 * i for i in range(n)]
+    g = torch.Generator().manual_seed(n + V)
+    logits = torch.randn(n, V, generator=g)
+    logits = ((logits * 64).round() / 64 if shape == "flat" else (logits * 2).round() / 2) + 0.0
+    words = (V + 31) // 32
+    allowed = torch.rand(words * 32, generator=g) < 0.3
+    allowed[0] = True
+    w = (allowed.view(words, 32).long() << torch.arange(32)).sum(1)
+    bits = torch.where(w >= 2 ** 31, w - 2 ** 32, w).to(torch.int32)
+    assert K._n.cuda_lib().cafd_sample_cluster(n, V, 148) == blocks
+    tok, st = (torch.full((n,), -7, dtype=torch.int32, device=dev) for _ in range(2))
+    rows = K.pack_sample_rows(params, positions, mask_word0=[0 if i % 3 == 0 else None for i in range(n)]).to(dev)
+    K.sample_rows(logits.to(dev), rows, tok, st, masks=bits.to(dev))
+    some = list(range(0, n, 11))
+    want, status = select_rows(logits[some], [params[i] for i in some], [positions[i] for i in some],
+                               [allowed[:V] if i % 3 == 0 else None for i in some])
+    assert not st.any() and tok[some].tolist() == want and status == [0] * len(some)
