@@ -49,7 +49,7 @@ struct SampleRow {          // 64 bytes
 enum : int { kSampleOk = 0, kSampleNonFinite = 1, kSampleEmptyMask = 2, kSampleBadParam = 3 };
 
 __device__ __forceinline__ uint32_t order_key(float x) {
-  const uint32_t b = __float_as_uint(x);
+  const uint32_t b = __float_as_uint(x + 0.0f);          // both zeros are one value
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 

@@ -89,7 +89,7 @@ def test_sample_rows_over_vocabularies(V, shape):
     if shape == "peaked":
         logits = logits * 2
         logits[:, :: max(1, V // 100)] += 12.0
-    logits = ((logits * 64).round() / 64 if shape != "ties" else (logits * 2).round() / 2) + 0.0      # no -0.0: the kernel's order puts it below 0.0
+    logits = (logits * 64).round() / 64 if shape != "ties" else (logits * 2).round() / 2              # zeros of both signs among them
     positions = [11 * i + V for i in range(n)]
     want, status = select_rows(logits, params, positions, [None] * n)
     tok = torch.full((n,), -7, dtype=torch.int32, device=dev)
@@ -111,7 +111,7 @@ def test_sample_many_rows(n, V, blocks, shape):
     positions = [7 * i for i in range(n)]
     g = torch.Generator().manual_seed(n + V)
     logits = torch.randn(n, V, generator=g)
-    logits = ((logits * 64).round() / 64 if shape == "flat" else (logits * 2).round() / 2) + 0.0
+    logits = (logits * 64).round() / 64 if shape == "flat" else (logits * 2).round() / 2
     words = (V + 31) // 32
     allowed = torch.rand(words * 32, generator=g) < 0.3
     allowed[0] = True
@@ -125,3 +125,23 @@ def test_sample_many_rows(n, V, blocks, shape):
     want, status = select_rows(logits[some], [params[i] for i in some], [positions[i] for i in some],
                                [allowed[:V] if i % 3 == 0 else None for i in some])
     assert not st.any() and tok[some].tolist() == want and status == [0] * len(some)
+
+
+@pytest.mark.parametrize("V", [40, 6000])
+def test_zeros_of_both_signs_are_one_value(V):
+    """The lowest id wins a tie also between 0.0 and -0.0: at the top-k boundary, in the nucleus and in the draw, with few tokens above the
+    line and with many."""
+    from cuteafd_b200.ops import kernels as K
+    from cuteafd_b200.runtime.sampling import SamplingParams, select_rows
+    dev = torch.device("cuda", 0)
+    kinds = [dict(top_k=5), dict(top_k=V - 7), dict(top_p=0.5), dict(), dict(min_p=0.9, top_k=3)]
+    params = [SamplingParams(temperature=1.0 + 0.1 * (i % 3), seed=i, **kinds[i % len(kinds)]) for i in range(40)]
+    logits = torch.zeros(40, V)
+    logits[:, ::2] = -0.0
+    logits[::2, V // 2] = 1.0
+    logits[:, V - 4:] = -3.0
+    positions = list(range(40))
+    want, status = select_rows(logits, params, positions, [None] * 40)
+    tok, st = (torch.full((40,), -7, dtype=torch.int32, device=dev) for _ in range(2))
+    K.sample_rows(logits.to(dev), K.pack_sample_rows(params, positions).to(dev), tok, st)
+    assert st.tolist() == status and tok.tolist() == want
