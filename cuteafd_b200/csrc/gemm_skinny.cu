@@ -50,7 +50,7 @@ struct SkinnyDev {
   void* out;
   const __nv_bfloat16* residual;
   const int* idx;                // grouped: expert of every entry
-  int* expert_count;             // grouped: optional, entries per expert
+  int* expert_count;             // grouped: optional, the step's entries per expert are added to it, as the plan of larger steps does
   int K, N, T, ldo, out_f32;
   int n_entries, row_div, E;     // grouped: entry e reads row e / row_div of x and writes row e of out
   int early;                     // the weights (and idx) are not written by the previous kernel of the stream
@@ -162,7 +162,7 @@ __device__ __forceinline__ void sk_plan(const SkinnyDev& p, SkinnyPlan& s, int* 
     if (tid == 31) { s.n_act = ia; s.off[ia] = static_cast<uint16_t>(in); }
   }
   if (p.expert_count && blockIdx.x == 0)
-    for (int e = tid; e < p.E; e += kSkThreads) p.expert_count[e] = cnt[e];
+    for (int e = tid; e < p.E; e += kSkThreads) p.expert_count[e] += cnt[e];
   __syncthreads();
   if (live) s.ent[off[mine] + place] = static_cast<uint8_t>(tid);
   __syncthreads();

@@ -59,7 +59,7 @@ def test_experts_of_a_step(T, top_k, E, I, H, spread):
     torch.cuda.synchronize()
     hbuf = torch.full((T * top_k, I), 3.0, dtype=torch.bfloat16, device=DEV)
     out = torch.full((T * top_k, H), 3.0, dtype=torch.bfloat16, device=DEV)
-    count = torch.full((E,), -1, dtype=torch.int32, device=DEV)
+    count = torch.arange(E, dtype=torch.int32, device=DEV)        # added to
     assert k.moe_skinny_ok(T * top_k, T, gate, x)
     k.moe_skinny(x, top_k, gate, up, idx, hbuf, expert_count=count)
     k.moe_skinny(hbuf, 1, down, None, idx, out, early=True)
@@ -73,7 +73,28 @@ def test_experts_of_a_step(T, top_k, E, I, H, spread):
         c, b = gate[ex].double() @ xe, up[ex].double() @ xe
         _close(hbuf[e], torch.nn.functional.silu(c) * b, 1.0 + c.abs() + b.abs())
         _close(out[e], down[ex].double() @ hbuf[e].double(), 1.0)
-    assert count.tolist() == torch.bincount(idx.flatten()[idx.flatten() < E], minlength=E).tolist()
+    assert (count.cpu() - torch.arange(E)).tolist() == torch.bincount(idx.flatten()[idx.flatten() < E], minlength=E).tolist()
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8"])
+def test_expert_counts_add_up_over_steps_of_any_size(fmt):
+    """A prompt-sized step, a few-row step and a prompt-sized one again: the exchange's counter holds the routes of all three."""
+    from cuteafd_b200.parallel.moe_exchange import ExchangeGeometry, LocalExchange
+    E, I, H, top_k = 16, 128, 256, 4
+    g = torch.Generator(device=DEV).manual_seed(3)
+    if fmt == "bf16":
+        ws = [torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((E, I, H), (E, I, H), (E, H, I))]
+    else:
+        ws = [_e4m3(s, g)[:2] for s in ((E, I, H), (E, I, H), (E, H, I))]
+    ex = LocalExchange(ExchangeGeometry(H, I, E, top_k, 64, 1), DEV)
+    seen = []
+    for T in (40, 5, 1, 40):
+        idx = torch.rand(T, E, device=DEV, generator=g).topk(top_k).indices.to(torch.int32)
+        ex.att.idx[:T], ex.att.w[:T] = idx, 1.0 / top_k
+        seen.append(idx.flatten())
+        x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+        (ex.forward if fmt == "bf16" else ex.forward_fp8)(x, None, {}, *ws, torch.empty_like(x))
+    assert torch.equal(ex.att.expert_count.long(), torch.bincount(torch.cat(seen).long(), minlength=E))
 
 
 def _e4m3(shape, g):
