@@ -179,6 +179,10 @@ __global__ void __launch_bounds__(kSkThreads, skinny_per_sm(kNT, kGB, kF8)) skin
   constexpr int kRows = kWR * (kDual ? 8 : 16);    // features of a block's tile
   constexpr int kRS = kNT * 8 + 1;
   constexpr int kElems = sk_elems(kF8);
+  // The tensor cores' fp32 sums lose a little with every product they take in: where registers are left, a batch's products are summed
+  // apart (2048 x 4096 at eight rows: 4.8e-7 -> 2.4e-7 off fp64, the split sums of the tcgen05 kernel 4.2e-7, at the same time; with more
+  // column tiles the sums' registers cost a tenth).  E4M3 blocks are summed apart anyway.
+  constexpr bool kApart = !kF8 && kGB > 2 && kNT == 1;
   __shared__ float red[2][kSkWarps * 16 * kRS];
   static_assert(sizeof(red) >= 2 * kSkMaxExperts * sizeof(int), "the sort of the routes works in the reduction buffer");
   __shared__ SkinnyPlan plan;
@@ -256,6 +260,7 @@ __global__ void __launch_bounds__(kSkThreads, skinny_per_sm(kNT, kGB, kF8)) skin
     float acc[kNT][4];
 #pragma unroll
     for (int nt = 0; nt < kNT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
     const int next = tile + gridDim.x;
     for (int b = 0; b < nb; ++b) {
       const bool last = b + 1 == nb;
@@ -308,6 +313,10 @@ __global__ void __launch_bounds__(kSkThreads, skinny_per_sm(kNT, kGB, kF8)) skin
         if (!last) fetch(i, b + 1, r0, r1);
         else if (next < n_tiles) fetch(i, 0, r0, r1);
       }
+      if constexpr (kApart) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { sum[e] += acc[0][e]; acc[0][e] = 0.f; }
+      }
     }
     // warps meet: buffer turn & 1 was last read two tiles ago, before the barrier of the tile between
     float* rb = red[turn & 1];
@@ -315,10 +324,11 @@ __global__ void __launch_bounds__(kSkThreads, skinny_per_sm(kNT, kGB, kF8)) skin
 #pragma unroll
     for (int nt = 0; nt < kNT; ++nt) {
       if (nt * 8 < cols) {
-        mine[g * kRS + nt * 8] = acc[nt][0];
-        mine[g * kRS + nt * 8 + 1] = acc[nt][1];
-        mine[(g + 8) * kRS + nt * 8] = acc[nt][2];
-        mine[(g + 8) * kRS + nt * 8 + 1] = acc[nt][3];
+        const float(&v)[4] = kApart ? sum : acc[nt];
+        mine[g * kRS + nt * 8] = v[0];
+        mine[g * kRS + nt * 8 + 1] = v[1];
+        mine[(g + 8) * kRS + nt * 8] = v[2];
+        mine[(g + 8) * kRS + nt * 8 + 1] = v[3];
       }
     }
     __syncthreads();

@@ -37,6 +37,26 @@ def test_dense_rows(T, N, K):
     _close(k.linear(xs, w, w_up=up, resident=True), torch.nn.functional.silu(c) * b, 1.0 + c.abs() + b.abs())
 
 
+@pytest.mark.parametrize("N,K", [(2048, 4096), (4096, 4096), (2176, 7168), (5120, 2048)])
+def test_sums_of_few_rows_lose_no_more_than_split_ones(N, K):
+    """fp32 results of up to eight rows are no further from fp64 than those of the kernel that the batch-invariant mode keeps, whose blocks
+    share K out (2-norms over eight draws: one and a half thousand to forty thousand values each, so the comparison is no coin's toss)."""
+    from cuteafd_b200.ops import kernels as k
+    off = []
+    for split in (0, 64):
+        k.set_fixed_kv_split(split)
+        try:
+            total = 0.0
+            for seed in range(8):
+                g = torch.Generator(device=DEV).manual_seed(seed)
+                x, w = (torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for s in ((seed + 1, K), (N, K)))
+                total += (k.linear(x, w, out_f32=True).double() - x.double() @ w.double().T).pow(2).sum().item()
+        finally:
+            k.set_fixed_kv_split(0)
+        off.append(total ** 0.5)
+    assert off[0] <= 1.02 * off[1]
+
+
 @pytest.mark.parametrize("T,top_k,E,I,H,spread", [(1, 8, 128, 768, 2048, "random"), (3, 2, 8, 64, 128, "one"), (8, 8, 256, 192, 1088, "random"),
                                                   (11, 8, 512, 256, 512, "random"), (12, 8, 128, 768, 2048, "random"), (12, 8, 16, 128, 2048, "one"),
                                                   (5, 4, 9, 128, 1024, "outside"), (12, 8, 9, 128, 1024, "same"), (8, 8, 9, 64, 128, "same")])
