@@ -81,6 +81,7 @@ typedef struct {
 
 int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream);
 int cafd_gemm_prompt_tile(int rows, int features, int num_sms);
+int cafd_gemm_few_rows(const cafd_gemm_args* a);     // whether cafd_gemm runs it on the few-row kernel
 
 // ---- greedy selection ----------------------------------------------------------------------------
 // out[t] = argmax over logits[t, 0:V] (row pitch ld, fp32); ties go to the lowest index and NaN is

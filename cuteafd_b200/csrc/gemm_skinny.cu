@@ -390,19 +390,26 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 using namespace cafd;
 
-// Whether cafd_gemm hands a dense product to this kernel.  Up to eight rows and K 4096 it was the faster one at every size measured
-// (2048 x 4096 to 37984 x 2048).  Longer K: one wave of tiles with four groups in flight (2176 x 7168: 11.8 against 13.3 us); beyond it
-// the rows of x don't stay in L1 (18432 x 7168 gate and up: 106 against 91 us).  Nine to sixteen rows: up to K 4096 and one wave of tiles
-// (5120 x 2048: 8.0 against 11.9 us; but 37984 x 2048: 42 against 38 us, 2176 x 7168: 19 against 14 us).  Up to 32 rows: a tile per SM at
-// most, where the other kernel cuts K nine ways and one block adds the parts (2048 x 4096: 13 against 31 us behind decode attention, 13
-// against 16 us behind a norm; 5120 x 2048: 15.6 against 15.1 us).
+// Whether cafd_gemm hands a dense product to this kernel.  Up to eight rows and K 4096 it is the faster one at every size measured up to some
+// 200 M weights (100 M of a gate and up pair): 2048 x 4096 to 65536 x 1024, 32000 x 4096 52 - 55 against 55 us, 10944 x 4096 pairs 40 - 43
+// against 42 us; beyond, the other kernel's copies keep more bytes in flight and its fill is not seen: 151936 x 2048 109 against 105 us,
+// 14336 x 4096 pairs 52 - 57 against 49 us.  Longer K: one wave of tiles with four groups in flight (2176 x 7168: 11.8 against 13.3 us);
+// beyond it the rows of x don't stay in L1 (18432 x 7168 gate and up: 106 against 91 us).  Nine to sixteen rows: up to K 4096 and one wave of
+// tiles (5120 x 2048: 8.0 against 11.9 us; but 37984 x 2048: 42 against 38 us, 2176 x 7168: 19 against 14 us).  Up to 32 rows: a tile per
+// SM at most, where the other kernel cuts K nine ways and one block adds the parts (2048 x 4096: 13 against 31 us behind decode attention;
+// behind a norm 15 against 17 us at 17 rows, 19 against 18 at 32; 5120 x 2048: 15.6 against 15.1 us).
 bool cafd::skinny_takes(const cafd_gemm_args* a) {
+  const int sms = a->num_sms > 0 ? a->num_sms : sm_count();
   const int tiles = (a->n_features + (a->dual ? 7 : 15)) / (a->dual ? 8 : 16);
-  const bool rows = a->x_rows <= 8 ? a->k <= 4096 || tiles <= 2 * 148 : a->x_rows <= kSkMaxRows && a->k <= 4096 && tiles <= (a->x_rows <= 16 ? 4 : 1) * 148;
+  const long long weights = static_cast<long long>(a->n_features) * a->k;        // of one of the two where there is a pair
+  const bool rows = a->x_rows <= 8 ? (a->k <= 4096 ? weights <= (a->dual ? 50 : 200) * 1000000ll : tiles <= 2 * sms)
+                                   : a->x_rows <= kSkMaxRows && a->k <= 4096 && tiles <= (a->x_rows <= 16 ? 4 : 1) * sms;
   return a->swap && !a->fp8 && a->x_rows > 0 && rows && a->k % sk_elems(false) == 0 && !a->tile_expert && !a->row_dst &&
          !a->row_scale && !a->wait_flag && !a->signal_flag && !a->rs_ranks && !a->n_signal_flags && !(a->dual && a->glu) &&
          !(a->dual && (!a->w1 || a->w1_row_offset)) && fixed_kv_split_tokens() == 0 && aligned16(a->w0) && aligned16(a->w1) && aligned16(a->x);
 }
+
+extern "C" int cafd_gemm_few_rows(const cafd_gemm_args* a) { return a && skinny_takes(a); }
 
 int cafd::skinny_dense(const cafd_gemm_args* a, cudaStream_t st) {
   SkinnyDev p{};
