@@ -345,13 +345,23 @@ def norm_route(h: torch.Tensor, ln_w: torch.Tensor | None, eps: float, router_w:
                                            int(group_score == "max"), _stream()), "norm_route")
 
 
-MOE_SKINNY_TOKENS = 12        # measured with plan, dispatch and combine: 12 tokens 140 against 145 us, 16 tokens 171 against 171 us
+# Tokens up to which a step's bf16 experts run on the few-row kernel, measured with plan, dispatch and combine against the tcgen05 kernel.
+# 128 experts of (768, 2048) at 12 tokens 131 against 155 us, 16 tokens 171 against 171; 56 of (1536, 4096) 266 against 290 us at 12.  Many
+# experts of large matrices give almost every route a matrix of its own, and from nine rows on, with two column tiles, it streams them more
+# slowly than the other kernel: 256 of (2048, 7168) at 8 tokens 759 against 810 us, at 10 1009 against 961; 128 of (1408, 4096) 299 against
+# 324 and 445 against 432 us at 8 and 12.
+MOE_SKINNY_TOKENS = 12
+MOE_SKINNY_TOKENS_LARGE = 8
+
+
+def moe_skinny_tokens(w: torch.Tensor) -> int:
+    return MOE_SKINNY_TOKENS_LARGE if w.shape[0] > 64 and w.shape[1] * w.shape[2] > 1 << 22 else MOE_SKINNY_TOKENS
 
 
 def moe_skinny_ok(n_entries: int, T: int, w: torch.Tensor, x: torch.Tensor) -> bool:
     """Whether a decode step's routed experts can take ``moe_skinny``: few rows, bf16, K in whole 64-element groups, and not in the
     batch-invariant mode (whose bits must not depend on the step's row count, so it keeps one kernel for all of them)."""
-    return (T <= MOE_SKINNY_TOKENS and n_entries <= _n.cuda_lib().cafd_moe_skinny_max_entries() and w.dtype == torch.bfloat16
+    return (T <= moe_skinny_tokens(w) and n_entries <= _n.cuda_lib().cafd_moe_skinny_max_entries() and w.dtype == torch.bfloat16
             and x.dtype == torch.bfloat16 and w.shape[0] <= 512 and w.shape[2] % 64 == 0 and fixed_kv_split() == 0)
 
 

@@ -2,6 +2,7 @@
 import ctypes as C
 
 import pytest
+import torch
 
 from cuteafd_b200._native import lib as _n
 
@@ -61,3 +62,12 @@ def test_few_row_products_leave_every_other_form_alone():
                dict(rs_ranks=2), dict(n_signal_flags=1), dict(w0=8), dict(x=8), dict(x_rows=0)):
         assert not _few(**{**ok, **{k: v for k, v in kw.items() if k in ok}}, **{k: v for k, v in kw.items() if k not in ok}), kw
     assert not _few(dual=True, glu=1, **ok) and not _few(dual=True, w1_row_offset=8, **ok)
+
+
+def test_few_row_experts_by_the_size_of_a_matrix():
+    from cuteafd_b200.ops import kernels as K
+    for (E, I, H), most in (((128, 768, 2048), 12), ((64, 1024, 2048), 12), ((56, 1536, 4096), 12), ((128, 1408, 4096), 8), ((256, 2048, 7168), 8), ((8, 14336, 4096), 12)):
+        for shape in ((E, I, H), (E, H, I)):
+            w = torch.empty(shape, dtype=torch.bfloat16, device="meta")
+            x = torch.empty(16, shape[2], dtype=torch.bfloat16, device="meta")
+            assert [K.moe_skinny_ok(2 * T, T, w, x) for T in range(1, 17)] == [T <= most for T in range(1, 17)]
