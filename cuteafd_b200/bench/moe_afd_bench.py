@@ -84,7 +84,7 @@ def main() -> None:
         epoch = worker.epoch
     dist.barrier()
     for T in Ts:
-        tile = plan_tile_rows("fp8" if a.fp8 else "bf16", min(T, geo.region().max_tokens), k, E)
+        tile = plan_tile_rows("fp8" if a.fp8 else "bf16", min(T, geo.region().max_tokens), k, E, I, H)
         if rank == 0:
             x = torch.randn(T, H, device=dev, generator=g).bfloat16()
             res = torch.randn(T, H, device=dev, generator=g).bfloat16()

@@ -16,7 +16,7 @@ import torch
 
 from ..config import ModelConfig
 from ..ops import kernels as K
-from ..parallel.moe_exchange import ExchangeGeometry, LocalExchange, pick_tile_rows
+from ..parallel.moe_exchange import ExchangeGeometry, LocalExchange
 
 PAGE = 64
 

@@ -36,7 +36,7 @@ import torch.distributed as dist
 from .._native import lib as _n
 from ..config import ModelConfig
 from ..ops import kernels as K
-from .moe_exchange import AttentionSide, ExchangeGeometry, ExpertSide, pick_tile_rows, plan_tile_rows, wire_fp8_ok
+from .moe_exchange import AttentionSide, ExchangeGeometry, ExpertSide, plan_tile_rows, wire_fp8_ok
 
 OP_STOP, OP_STEPS, OP_TIMED, OP_SYNC = 0, 1, 2, 3
 
@@ -178,7 +178,7 @@ class RemoteExchange:
         self._pending = (T, waves)
         dslot = self.layer * self.dflag_stride + self.source * n       # this source's dispatch flags of the layer
         if len(waves) == 1:
-            tile_rows = tile_rows or plan_tile_rows(self.expert_format, T, g.top_k, g.num_experts)
+            tile_rows = tile_rows or plan_tile_rows(self.expert_format, T, g.top_k, g.num_experts, g.expert_ffn, g.hidden)
             self.att.dispatch(x, logits, route_kw, tile_rows, dslot, self.epoch, wire_fp8=self._wire(self.att, tile_rows))
             return
         assert logits is not None, "fused routing is for single-wave steps"
@@ -186,7 +186,7 @@ class RemoteExchange:
         for w, (a, b) in enumerate(waves):
             side = self.sides[w]
             side.combine = self.combine[a * k:]
-            tr = plan_tile_rows(self.expert_format, b - a, k, g.num_experts)
+            tr = plan_tile_rows(self.expert_format, b - a, k, g.num_experts, g.expert_ffn, g.hidden)
             side.dispatch(x[a:b], logits[a:b], route_kw, tr, dslot + w, self.epoch, wire_fp8=self._wire(side, tr))
 
     def finish(self, out, *, shared=None, residual=None, norm_w=None, eps=0.0, x_out=None):
@@ -406,7 +406,7 @@ class ExpertWorker:
                     flag = self.cflags_ptrs[a] + 4 * ((l * n + w) * _n.MAX_RANKS + self.er)
                     side = self.sides[a][w]
                     combine_ptr = self.combine_ptrs[a] + t0 * g.top_k * g.hidden * 2
-                    tile_rows = plan_tile_rows(fmt, t1 - t0, g.top_k, g.num_experts)
+                    tile_rows = plan_tile_rows(fmt, t1 - t0, g.top_k, g.num_experts, g.expert_ffn, g.hidden)
                     if fmt == "fp8":                 # E4M3 values + 128x128 block scales
                         rows = min(side.geo.max_rows, (t1 - t0) * g.top_k + (hi - lo) * tile_rows)
                         side.run_fp8(wg, wu, wd, tile_rows, rows, dslot, self.epochs[a], combine_ptr, flag, wait=True,

@@ -23,25 +23,45 @@ from ..ops import kernels as K
 from ..ref.split import expert_range
 
 
-def pick_tile_rows(T: int, top_k: int, num_experts: int) -> int:
-    """Row tile of bf16 experts by the mean segment length.  Measured over the whole exchange (128 experts of (768, 2048), top-8), tiles of
-    16 / 32 / 64 / 128 rows, us: 128 tokens 242 / 285 / 383 / 305, 256 tokens 272 / 293 / 391 / 304, 320 tokens 302 / 297 / 395 / 303,
-    384 tokens 325 / 307 / 399 / 303, 512 tokens 380 / 355 / 406 / 313: weights on the M side while a segment is about one narrow tile,
-    tokens on it from there on."""
+def pick_tile_rows(T: int, top_k: int, num_experts: int, ffn: int = 0, hidden: int = 0) -> int:
+    """Row tile of bf16 experts of (``ffn``, ``hidden``) by the mean segment length.  Tiles of 16 and 32 rows keep the weights on the M side
+    and read them again for every tile of a segment; tiles of 128 read them once, are padded to 128 rows and cut nothing over K.  Timed over
+    the whole exchange for 8 experts of (14336, 4096), 56 and 64 of (512, 1024) to (1536, 4096), 128 of (768, 2048) and (1408, 4096), 256
+    and 384 of (2048, 7168), us at a mean of about 9 / 12 / 16 / 20 / 24 / 32 rows:
+
+    ======================  =====================================  =====================================  ====================================
+    experts                 tiles of 16                            32                                     128
+    ======================  =====================================  =====================================  ====================================
+    64 x (1024, 2048)       179 / 179 / 202 / 223 / 221 / 276      196 / 197 / 191 / 201 / 202 / 243      229 / 230 / 225 / 229 / 232 / 226
+    56 x (1536, 4096)       381 / 403 / 424 / 487 / 531 / 616      397 / 397 / 400 / 400 / 397 / 448      413 / 422 / 423 / 426 / 424 / 423
+    8 x (14336, 4096)       488 / 474 / 556 / 642 / 688 / 731      501 / 506 / 508 / 501 / 504 / 565      523 / 525 / 526 / 522 / 529 / 534
+    128 x (768, 2048)       241 / 250 / 274 / 285 / 328 / 382      284 / 293 / 297 / 293 / 308 / 358      305 / 313 / 317 / 317 / 309 / 317
+    128 x (1408, 4096)      738 / 746 / 838 / 957 / 1061 / 1231    789 / 783 / 792 / 797 / 816 / 944      792 / 789 / 795 / 799 / 799 / 806
+    256 x (2048, 7168)      3599 / 3971 / 4881 / 6120 / 5436 / -   3792 / 3809 / 3815 / 3855 / 3892 / -   3602 / 3609 / 3628 / 3605 / 3622 / -
+    ======================  =====================================  =====================================  ====================================
+
+    A second reading of 16-row tiles comes out of L2 only while the layer's matrices are small, and a few experts give tiles of 128 rows
+    too few blocks to fill the last wave.  64-row tiles were the slowest form everywhere."""
     avg = T * top_k / max(1, num_experts)
-    return 16 if avg <= 16 else 32 if avg <= 20 else 128
+    size = ffn * hidden
+    if num_experts * -(-ffn // 128) >= 16 * 148:            # sixteen waves of fc1 tiles: nothing stays in L2 between tiles
+        return 16 if avg <= 11 else 32 if avg <= 20 else 128
+    if avg <= (16 if size < 1 << 21 else 15 if size <= 1 << 22 else 13):
+        return 16
+    return 32 if avg <= (26 if num_experts <= 64 else 22) else 128
 
 
-def plan_tile_rows(fmt: str, T: int, top_k: int, num_experts: int) -> int:
+def plan_tile_rows(fmt: str, T: int, top_k: int, num_experts: int, ffn: int = 0, hidden: int = 0) -> int:
     """Row tile of a step's expert segments for experts stored as ``fmt``.  Both halves of an exchange derive it from
     the same arguments: the planner pads every expert's segment to it and the grouped GEMMs walk the tiles with it.
     Quantised experts read their packed weights directly up to 64-row tiles; 128-row tiles mean the layer's experts are
-    expanded to bf16 first, which only pays once every expert sees at least 64 rows on average."""
+    expanded to bf16 first, which only pays once every expert sees at least 64 rows on average.  32-bit experts ("fp32") are
+    multiplied in blocks of 64 rows, padding included."""
     if fmt == "bf16":
-        return pick_tile_rows(T, top_k, num_experts)
+        return pick_tile_rows(T, top_k, num_experts, ffn, hidden)
     avg = T * top_k / max(1, num_experts)
     t = 16 if avg <= 8 else 32 if avg <= 24 else 64
-    return 128 if t == 64 and avg >= 64 else t
+    return 128 if t == 64 and avg >= (48 if fmt == "fp32" else 64) else t
 
 
 def wire_fp8_ok(geo: "ExchangeGeometry", tile_rows: int) -> bool:
@@ -323,9 +343,13 @@ class LocalExchange:
         if self.skinny(x, w_gate, w_down):
             self._run_skinny(x, logits, route_kw, w_gate, w_up, w_down)
             return
-        tile_rows = pick_tile_rows(T, g.top_k, g.num_experts)
+        tile_rows = self._tile_rows(x)
         self.att.dispatch(x, logits, route_kw, tile_rows, 0, self.epoch)
         self.exp.run(w_gate, w_up, w_down, tile_rows, 0, self.epoch, self.att.combine.data_ptr(), None, wait=False)
+
+    def _tile_rows(self, x: torch.Tensor) -> int:
+        g = self.geo
+        return plan_tile_rows("fp32" if x.dtype == torch.float32 else "bf16", x.shape[0], g.top_k, g.num_experts, g.expert_ffn, g.hidden)
 
     def forward(self, x: torch.Tensor, logits: torch.Tensor, route_kw: dict, w_gate: torch.Tensor, w_up: torch.Tensor,
                 w_down: torch.Tensor, out: torch.Tensor, *, shared: torch.Tensor | None = None,
@@ -339,7 +363,7 @@ class LocalExchange:
             self._run_skinny(x, logits, route_kw, w_gate, w_up, w_down)
             return self.att.combine_into(out, T, 0, self.epoch, shared=shared, residual=residual, wait=False, norm_w=norm_w, eps=eps,
                                          x_out=x_out)
-        tile_rows = tile_rows or pick_tile_rows(T, g.top_k, g.num_experts)
+        tile_rows = tile_rows or self._tile_rows(x)
         self.att.dispatch(x, logits, route_kw, tile_rows, 0, self.epoch)
         self.exp.run(w_gate, w_up, w_down, tile_rows, 0, self.epoch, self.att.combine.data_ptr(), None, wait=False)
         return self.att.combine_into(out, T, 0, self.epoch, shared=shared, residual=residual, wait=False, norm_w=norm_w,

@@ -459,7 +459,7 @@ def cuda_compute(stack_of, lo: int, device, expert_ffn: int):
         n_exp, n, H = gate.shape[0], len(row), x.shape[1]
         if n == 0:
             return torch.zeros(0, H, dtype=torch.float32)
-        tile = pick_tile_rows(max(1, n // max(1, len(np.unique(expert)))), 1, 1)
+        tile = pick_tile_rows(n, 1, len(np.unique(expert)), expert_ffn, H)
         order = np.argsort(expert, kind="stable")
         local = expert[order].astype(np.int64) - lo
         counts = np.bincount(local, minlength=n_exp)

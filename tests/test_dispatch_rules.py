@@ -71,3 +71,29 @@ def test_few_row_experts_by_the_size_of_a_matrix():
             w = torch.empty(shape, dtype=torch.bfloat16, device="meta")
             x = torch.empty(16, shape[2], dtype=torch.bfloat16, device="meta")
             assert [K.moe_skinny_ok(2 * T, T, w, x) for T in range(1, 17)] == [T <= most for T in range(1, 17)]
+
+
+# us of a whole exchange with row tiles of 16 / 32 / 64 / 128, by geometry and mean segment length
+TILE_TIMES = {
+    (64, 1024, 2048): {9: (179, 196, 251, 229), 12: (179, 197, 252, 230), 15: (190, 198, 245, 225), 16: (202, 191, 246, 225), 20: (223, 201, 255, 229), 24: (221, 202, 257, 232),
+                       26: (247, 206, 258, 231), 32: (276, 243, 249, 226), 48: (352, 273, 262, 228)},
+    (56, 1536, 4096): {8.04: (380, 398, 462, 419), 11: (375, 399, 464, 420), 16: (424, 400, 470, 423), 20.1: (487, 400, 474, 426), 24: (531, 397, 477, 424), 26: (531, 396, 483, 426), 32: (616, 448, 479, 423)},
+    (8, 14336, 4096): {10: (488, 501, 536, 523), 14: (540, 504, 533, 519), 16: (556, 508, 535, 526), 21: (668, 506, 538, 529), 24: (688, 504, 539, 529), 26: (688, 509, 539, 529), 44: (987, 681, 538, 527)},
+    (128, 768, 2048): {9: (241, 284, 381, 305), 12: (250, 293, 395, 313), 16: (274, 297, 396, 317), 21: (311, 301, 401, 317), 26: (328, 308, 400, 309), 32: (382, 358, 413, 317)},
+    (128, 1408, 4096): {9: (738, 789, 966, 792), 11: (732, 791, 953, 785), 16: (838, 792, 963, 795), 22: (1025, 789, 983, 800), 24: (1061, 816, 975, 799), 32: (1231, 944, 995, 806)},
+    (256, 2048, 7168): {8: (3860, 4028, 4306, 3570), 16: (4881, 3815, 4328, 3628), 20: (6120, 3855, 4353, 3605), 24: (5436, 3892, 4434, 3622), 32: (7534, 4247, 4413, 3625)},
+}
+
+
+def test_row_tiles_are_the_faster_ones_at_every_geometry_measured():
+    """Within 3 % of the better of the two rules that knew the mean segment alone (16 / 32 / 64 / 128 up to 8 / 24 / 48 rows, and 16 / 32 / 128
+    up to 16 / 20), which lost up to a third of each other's time."""
+    from cuteafd_b200.parallel.moe_exchange import pick_tile_rows, plan_tile_rows
+    for (E, ffn, hidden), rows in TILE_TIMES.items():
+        for avg, us in rows.items():
+            took = dict(zip((16, 32, 64, 128), us))
+            a, b = 16 if avg <= 8 else 32 if avg <= 24 else 64 if avg <= 48 else 128, 16 if avg <= 16 else 32 if avg <= 20 else 128
+            got = pick_tile_rows(round(avg * E), 1, E, ffn, hidden)
+            assert took[got] <= 1.03 * min(took[a], took[b]), (E, ffn, hidden, avg, got)
+            assert plan_tile_rows("bf16", round(avg * E), 1, E, ffn, hidden) == got
+    assert [plan_tile_rows("fp32", 16 * n, 1, 16) for n in (8, 9, 24, 25, 47, 48)] == [16, 32, 32, 64, 64, 128]
