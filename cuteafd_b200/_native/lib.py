@@ -208,6 +208,7 @@ def cuda_lib():
         _sig(lib, "cafd_gemm_prompt_tile", [I, I, I])
         _sig(lib, "cafd_gemm_few_rows", [C.POINTER(GemmArgs)])
         _sig(lib, "cafd_sample_cluster", [I, I, I])
+        _sig(lib, "cafd_rope_heads_per_warp", [I, I, I])
         _sig(lib, "cafd_moe_skinny", [P, I, P, P, P, P, P, I, I, I, I, I, P, I, P, I, I, P])
         _sig(lib, "cafd_linear_w8", [P, I, P, P, P, P, I, I, P, I, P, I, I, P])
         _sig(lib, "cafd_moe_skinny_max_entries", [])

@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* __restrict__ 
 // q_out [T, Hq, D]; K/V pages [num_pages, page, Hkv, D]; slot[t] = page * page_size + offset.
 // Rounding points follow the oracle: norm -> bf16 -> rope (fp32) -> bf16.
 // kHeads: heads of one token that a warp does.  The angles are the expensive part (two sincosf at large arguments per lane) and are the
-// token's, not the head's, so a prompt chunk takes eight heads per warp, all their loads in flight at once: 8192 tokens of 32 + 2 x 4
-// heads 96 -> 60 us.  A decode step, short of warps, takes one.
+// token's, not the head's, so a prompt chunk takes up to eight heads per warp, a token's heads shared out evenly and all loads of a warp in
+// flight at once: 8192 tokens of 32 + 2 x 4 heads 87 -> 48 us.  A step short of warps takes one.
 template <int kHeads>
 __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __restrict__ qkv,
                                                          const __nv_bfloat16* __restrict__ q_norm_w,
@@ -111,17 +111,17 @@ __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __
   pdl_wait();
   pdl_trigger();
   constexpr int D = 128;
-  const int heads = Hq + 2 * Hkv, chunks = (heads + kHeads - 1) / kHeads;
+  const int heads = Hq + 2 * Hkv, chunks = (heads + kHeads - 1) / kHeads, per = kHeads == 1 ? 1 : (heads + chunks - 1) / chunks;
   const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (gw >= T * chunks) return;
   const int t = gw / chunks;
-  const int h_lo = (gw % chunks) * kHeads;
+  const int h_lo = (gw % chunks) * per, h_hi = min(heads, h_lo + per);
   const int lane = threadIdx.x & 31;
   // lane holds elements {2l, 2l+1} and {64+2l, 64+2l+1}
   uint32_t ra_[kHeads], rb_[kHeads];
 #pragma unroll
   for (int i = 0; i < kHeads; ++i) {
-    const int h = min(h_lo + i, heads - 1);
+    const int h = min(h_lo + i, h_hi - 1);
     const __nv_bfloat16* src = qkv + (static_cast<size_t>(t) * heads + h) * D;
     ra_[i] = *reinterpret_cast<const uint32_t*>(src + 2 * lane);
     rb_[i] = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane);
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __
 #pragma unroll
   for (int i = 0; i < kHeads; ++i) {
     const int h = h_lo + i;
-    if (h >= heads) return;
+    if (h >= h_hi) return;
     uint32_t a = ra_[i], b = rb_[i];
     if (bias) {
       const uint32_t ba = *reinterpret_cast<const uint32_t*>(bias + h * D + 2 * lane);
@@ -302,6 +302,13 @@ extern "C" int cafd_rmsnorm(const void* x, void* residual, const void* w, void* 
   return static_cast<int>(cudaGetLastError());
 }
 
+// Most heads per warp of a step's rotation: eight once that leaves twelve warps per SM.  Below, one head per warp is the faster form (8 + 2 x 1
+// heads, 300 tokens: 2.8 us against 4.5 with eight heads and two; 32 + 2 x 4, 256: 4.2 against 4.7), above it the shared angles are
+// (32 + 2 x 4, 512: 5.3 against 6.6; 1 + 2 x 1, 2048: 3.0 against 3.4).
+extern "C" int cafd_rope_heads_per_warp(int T, int heads, int num_sms) {
+  return static_cast<long long>(T) * ((heads + 7) / 8) >= 12ll * num_sms ? 8 : 1;
+}
+
 extern "C" int cafd_qk_rope_kv(const void* qkv, const void* q_norm_w, const void* k_norm_w, const float* inv_freq,
                                const int* positions, const int* slots, void* q_out, void* k_cache, void* v_cache,
                                int T, int Hq, int Hkv, int D, float eps, int interleaved, const void* bias, int rot,
@@ -309,7 +316,10 @@ extern "C" int cafd_qk_rope_kv(const void* qkv, const void* q_norm_w, const void
   if (T <= 0) return 0;
   if (D != 128 || (rot != 128 && rot != 64)) return -10;
   const int heads = Hq + 2 * Hkv;
-  const bool many = T >= 256;                // about two blocks of eight-head warps per SM
+  int dev = 0, sms = 0;
+  CAFD_CHECK_CUDA(cudaGetDevice(&dev));
+  CAFD_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool many = cafd_rope_heads_per_warp(T, heads, sms) == 8;
   const int warps = T * (many ? (heads + 7) / 8 : heads);
   const int blocks = (warps + 3) / 4;
   launch_pdl(many ? qk_rope_kv_kernel<8> : qk_rope_kv_kernel<1>, dim3(blocks), dim3(128), 0, static_cast<cudaStream_t>(s), 

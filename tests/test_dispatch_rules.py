@@ -97,3 +97,12 @@ def test_row_tiles_are_the_faster_ones_at_every_geometry_measured():
             assert took[got] <= 1.03 * min(took[a], took[b]), (E, ffn, hidden, avg, got)
             assert plan_tile_rows("bf16", round(avg * E), 1, E, ffn, hidden) == got
     assert [plan_tile_rows("fp32", 16 * n, 1, 16) for n in (8, 9, 24, 25, 47, 48)] == [16, 32, 32, 64, 64, 128]
+
+
+def test_rotation_shares_angles_once_there_are_warps_enough():
+    """By the warps that the step has, not by its tokens: a shard with few heads needs more of them."""
+    per = _n.cuda_lib().cafd_rope_heads_per_warp
+    for sms in (40, 148):
+        for heads in (3, 6, 10, 40, 112):
+            T = -(-12 * sms // -(-heads // 8))
+            assert per(1, heads, sms) == per(T - 1, heads, sms) == 1 and per(T, heads, sms) == per(1 << 20, heads, sms) == 8

@@ -36,24 +36,28 @@ def test_projections_do_not_depend_on_the_tile_width(K):
     assert k._n.cuda_lib().cafd_gemm_prompt_tile(2300, N, k.num_sms()) == 256 and set(widths) == {64, 128, 256}
 
 
-@pytest.mark.parametrize("Hq,Hkv", [(32, 4), (8, 2), (5, 1)])
+@pytest.mark.parametrize("Hq,Hkv", [(32, 4), (8, 2), (5, 1), (13, 2)])
 @pytest.mark.parametrize("interleaved,rot,bias", [(False, 128, False), (True, 128, True), (False, 64, False), (True, 64, False)])
 def test_rope_of_a_prompt_is_that_of_its_tokens(Hq, Hkv, interleaved, rot, bias):
-    """Eight heads per warp (from 256 tokens on) and one: the same bits, heads past a multiple of eight and dropped slots included."""
+    """Up to eight heads per warp and one: the same bits, head counts that share out evenly and not, dropped slots included."""
     from cuteafd_b200.ops import kernels as k
-    T, D = 300, 128
+    heads, D = Hq + 2 * Hkv, 128
+    T = 12 * k.num_sms() // -(-heads // 8) + 11
+    per = k._n.cuda_lib().cafd_rope_heads_per_warp
+    assert per(T, heads, k.num_sms()) == 8 and per(100, heads, k.num_sms()) == 1
     g = torch.Generator(device=DEV).manual_seed(Hq)
     qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, generator=g).to(torch.bfloat16)
     qn, kn = (1 + torch.rand(D, device=DEV, generator=g)).to(torch.bfloat16), (1 + torch.rand(D, device=DEV, generator=g)).to(torch.bfloat16)
     b = torch.randn((Hq + 2 * Hkv) * D, device=DEV, generator=g).to(torch.bfloat16) if bias else None
     inv = (1e6 ** (-torch.arange(0, rot, 2, device=DEV).float() / rot)).contiguous()
     pos = torch.arange(8000, 8000 + T, dtype=torch.int32, device=DEV)
-    slots = torch.randperm(6 * 64, device=DEV, generator=g)[:T].to(torch.int32)
+    pages = T // 64 + 2
+    slots = torch.randperm(pages * 64, device=DEV, generator=g)[:T].to(torch.int32)
     slots[7] = -1
     outs = []
     for step in (T, 100):
         q = torch.zeros(T, Hq, D, dtype=torch.bfloat16, device=DEV)
-        kc, vc = (torch.zeros(6, Hkv, 64, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        kc, vc = (torch.zeros(pages, Hkv, 64, D, dtype=torch.bfloat16, device=DEV) for _ in range(2))
         for a in range(0, T, step):
             k.qk_rope_kv(qkv[a:a + step], qn, kn, inv, pos[a:a + step], slots[a:a + step], q[a:a + step], kc, vc, Hq, Hkv, D, 1e-6, interleaved, bias=b)
         outs.append((q, kc, vc))
