@@ -354,8 +354,12 @@ __device__ __forceinline__ float ld_partial(const float* p) {
 
 // One block per (tile, kv head, row; with two maps row pair): thread d walks the splits in order for its output element.  The splits'
 // maxima are read once, a split per lane, and their factors handed round, so that the walk is independent loads (32 splits of one row:
-// 8.1 us behind the partials when every thread read every maximum twice, one after the other, now 7.3).
-template <int kMaps, bool kTurn = false>
+// 8.1 us behind the partials when every thread read every maximum twice, one after the other, now 7.3).  kFew: up to four splits, of which
+// every thread reads all there is at once; handing factors round costs more than it saves there (attention of 32 rows of 500 tokens in two
+// splits 18.8 -> 20.0 us), and both walks in one kernel made the long one a tenth slower.  They do the same sums, so a row's bits don't
+// depend on how many empty splits follow its own.
+constexpr int kFewSplits = 4;
+template <int kMaps, bool kTurn, bool kFew>
 __global__ void __launch_bounds__(128) attn_merge_kernel(const float* __restrict__ partial,
                                                          const int* __restrict__ q_start,
                                                          __nv_bfloat16* __restrict__ out, int Hq, int Hkv,
@@ -376,25 +380,43 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const float* __restrict
   for (int m = 0; m < kMaps; ++m) {
     const int row = r * kMaps + m;
     const float* stat = base + 16 * kD + row;
-    float M = -INFINITY;
-    for (int s = lane; s < splits; s += 32) M = fmaxf(M, __ldg(stat + s * kPartialFloats));
-    M = warp_max(M);
-    float L = 0.f, O = 0.f;
-    for (int s0 = 0; s0 < splits; s0 += 32) {
-      const int s = min(s0 + lane, splits - 1);
-      const float mx = __ldg(stat + s * kPartialFloats);
-      const float f = (s0 + lane >= splits || mx == -INFINITY) ? 0.f : exp2f(mx - M);
-      const float lf = __ldg(stat + s * kPartialFloats + 16) * f;
-      const float* o = base + row * kD + d + static_cast<size_t>(s0) * kPartialFloats;
-      const int n = min(32, splits - s0);
-      for (int i0 = 0; i0 < n; i0 += 16) {
-        float part[16];
+    float M = -INFINITY, L = 0.f, O = 0.f;
+    if constexpr (kFew) {
+      float mx[kFewSplits], l[kFewSplits], part[kFewSplits];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) part[i] = i0 + i < n ? ld_partial(o + static_cast<size_t>(i0 + i) * kPartialFloats) : 0.f;
+      for (int s = 0; s < kFewSplits; ++s) {
+        const int at = min(s, splits - 1) * kPartialFloats;
+        mx[s] = ld_partial(stat + at);
+        l[s] = ld_partial(stat + at + 16);
+        part[s] = ld_partial(base + row * kD + d + at);
+      }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          L += __shfl_sync(0xffffffffu, lf, (i0 + i) & 31);            // zero factors past the last split
-          O += part[i] * __shfl_sync(0xffffffffu, f, (i0 + i) & 31);
+      for (int s = 0; s < kFewSplits; ++s) M = fmaxf(M, mx[s]);
+#pragma unroll
+      for (int s = 0; s < kFewSplits; ++s) {
+        const float f = (s >= splits || mx[s] == -INFINITY) ? 0.f : exp2f(mx[s] - M);
+        L = __fadd_rn(L, __fmul_rn(l[s], f));
+        O = __fmaf_rn(part[s], f, O);
+      }
+    } else {
+      for (int s = lane; s < splits; s += 32) M = fmaxf(M, __ldg(stat + s * kPartialFloats));
+      M = warp_max(M);
+      for (int s0 = 0; s0 < splits; s0 += 32) {
+        const int s = min(s0 + lane, splits - 1);
+        const float mx = __ldg(stat + s * kPartialFloats);
+        const float f = (s0 + lane >= splits || mx == -INFINITY) ? 0.f : exp2f(mx - M);
+        const float lf = __fmul_rn(__ldg(stat + s * kPartialFloats + 16), f);
+        const float* o = base + row * kD + d + static_cast<size_t>(s0) * kPartialFloats;
+        const int n = min(32, splits - s0);
+        for (int i0 = 0; i0 < n; i0 += 16) {
+          float part[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) part[i] = i0 + i < n ? ld_partial(o + static_cast<size_t>(i0 + i) * kPartialFloats) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            L = __fadd_rn(L, __shfl_sync(0xffffffffu, lf, (i0 + i) & 31));            // zero factors past the last split
+            O = __fmaf_rn(part[i], __shfl_sync(0xffffffffu, f, (i0 + i) & 31), O);
+          }
         }
       }
     }
@@ -463,7 +485,10 @@ extern "C" int cafd_attn_decode(const void* q, const void* k_cache, const void* 
       window, fixed_kv_split_tokens() / kPage, AttnPeers{}, ex);
   if (splits > 1) {
     dim3 g2(num_seqs * tiles_per_seq, Hkv, 16 / maps);
-    auto merge = maps == 2 ? attn_merge_kernel<2> : turn ? attn_merge_kernel<1, true> : attn_merge_kernel<1>;
+    const bool few = splits <= kFewSplits;
+    auto merge = maps == 2 ? (few ? attn_merge_kernel<2, false, true> : attn_merge_kernel<2, false, false>)
+               : turn      ? (few ? attn_merge_kernel<1, true, true> : attn_merge_kernel<1, true, false>)
+                           : (few ? attn_merge_kernel<1, false, true> : attn_merge_kernel<1, false, false>);
     launch_pdl(merge, g2, dim3(128), 0, st, scratch, q_start, static_cast<__nv_bfloat16*>(out), Hq, Hkv, tiles_per_seq, splits, ex);
   }
   return static_cast<int>(cudaGetLastError());
@@ -515,7 +540,7 @@ extern "C" int cafd_attn_merge(const float* scratch, const int* q_start, void* o
   const int q_per_tile = 16 / group;
   const int tiles_per_seq = (max_q_len + q_per_tile - 1) / q_per_tile;
   dim3 g2(num_seqs * tiles_per_seq, Hkv, 16);
-  launch_pdl(attn_merge_kernel<1>, g2, dim3(128), 0, static_cast<cudaStream_t>(s), scratch, q_start, static_cast<__nv_bfloat16*>(out),
+  launch_pdl(total_splits <= kFewSplits ? attn_merge_kernel<1, false, true> : attn_merge_kernel<1, false, false>, g2, dim3(128), 0, static_cast<cudaStream_t>(s), scratch, q_start, static_cast<__nv_bfloat16*>(out),
              Hq, Hkv, tiles_per_seq, total_splits, AttnExtras{0, Hq * kD});
   return static_cast<int>(cudaGetLastError());
 }

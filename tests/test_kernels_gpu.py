@@ -235,6 +235,26 @@ def test_attn_decode(K, lens, qlens, splits):
         o += qlens[s]
 
 
+@pytest.mark.parametrize("splits", [5, 8, 32, 40])
+def test_attn_decode_bits_do_not_depend_on_empty_splits(K, splits):
+    """Fixed splits of 64 tokens over rows of up to four: merged by the walk for few splits and by the one for many, the same bits."""
+    Hq, Hkv, D, lens = 32, 4, 128, [256, 1, 190, 64, 130]
+    S = len(lens)
+    kc, vc, table, _ = _paged_kv(S, lens, Hkv, D)
+    q = bf(S, Hq, D, seed=99)
+    q_start = torch.arange(S + 1, dtype=torch.int32, device=dev())
+    seq_lens = torch.tensor(lens, dtype=torch.int32, device=dev())
+    outs = []
+    K.set_fixed_kv_split(64)
+    try:
+        for n in (4, splits):
+            scratch = torch.empty(K.attn_decode_scratch_floats(S, 1, Hq, Hkv, n), dtype=torch.float32, device=dev())
+            outs.append(K.attn_decode(q, kc, vc, table, seq_lens, q_start, torch.zeros_like(q), scratch, 1, n).clone())
+    finally:
+        K.set_fixed_kv_split(0)
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("lens,qlens", [([128], [128]), ([300], [300]), ([1000], [200]), ([517, 130], [517, 66]),
                                         ([2048], [2048])])
 def test_attn_prefill(K, lens, qlens):
