@@ -27,6 +27,7 @@
 // kernel, so the batch-invariant mode, which promises the same bits at any row count, stays on the tcgen05 kernel.
 #include "cafd_api.h"
 #include "common.cuh"
+#include <atomic>
 
 namespace cafd {
 
@@ -358,10 +359,17 @@ template <int kNT, int kWK, int kGB, bool kDual, bool kGrouped, bool kF8>
 static int launch_skinny(const SkinnyDev& p, long long tiles, int sms, cudaStream_t st) {
   // Left to itself the driver sizes shared memory for this kernel alone.  The first blocks then start on SMs that the previous
   // kernel still holds at another split, a fourth block finds no room until an SM is drained, and its share of the tiles runs after
-  // everybody else's (fc1 of eight rows: 83 us in the chain, 55 us alone).  64 KB hold four blocks and leave the rest to L1.
-  static const cudaError_t carve = cudaFuncSetAttribute(skinny_kernel<kNT, kWK, kGB, kDual, kGrouped, kF8>,
-                                                        cudaFuncAttributePreferredSharedMemoryCarveout, 28);
-  CAFD_CHECK_CUDA(carve);
+  // everybody else's (fc1 of eight rows: 83 us in the chain, 55 us alone).  64 KB hold four blocks of one column
+  // tile, three of two and one of four (whose products have at most one tile per SM) and leave the rest to L1.  The attribute is the
+  // device's: it is set once on each.
+  static std::atomic<unsigned long long> set{0};
+  int dev = 0;
+  CAFD_CHECK_CUDA(cudaGetDevice(&dev));
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev > 63 || !(set.load(std::memory_order_relaxed) & bit)) {
+    CAFD_CHECK_CUDA(cudaFuncSetAttribute(skinny_kernel<kNT, kWK, kGB, kDual, kGrouped, kF8>, cudaFuncAttributePreferredSharedMemoryCarveout, 28));
+    set.fetch_or(bit, std::memory_order_relaxed);
+  }
   const long long most = static_cast<long long>(skinny_per_sm(kNT, kGB, kF8)) * sms;
   launch_pdl(skinny_kernel<kNT, kWK, kGB, kDual, kGrouped, kF8>, dim3(static_cast<unsigned>(tiles < most ? tiles : most)), dim3(kSkThreads), 0, st, p);
   return static_cast<int>(cudaGetLastError());
