@@ -328,13 +328,13 @@ class GqaMoeEngine:
             return K.linear_fp8(xq, xs, w[0], w[1], out, w_up=u[0] if u else None, ws_up=u[1] if u else None, residual=residual)
         return K.linear(x, getattr(L, name), out=out, w_up=getattr(L, up) if up else None, residual=residual, resident=True)
 
+    FEW_ROW_LAUNCHES = 3            # an exchange without plan and dispatch: fc1, fc2, combine
+
     def _exchange_launches(self, T: int) -> int:
         """Kernels one bf16 exchange launches for T tokens: plan (with the dispatch folded in for very small steps, three
         launches wide from 8192 entries on), dispatch, fc1, fc2, combine."""
         from ..parallel.moe_exchange import AttentionSide as A
         n = T * self.cfg.top_k
-        if T <= K.MOE_SKINNY_TOKENS and n <= 256 and not self.fixed_kv_split and isinstance(self.moe, LocalExchange):
-            return 3                                                 # fc1, fc2, combine
         fused = n <= A.FUSED_DISPATCH_ROWS and n * self.cfg.hidden * 2 <= A.FUSED_DISPATCH_BYTES
         return (4 if fused else 5) + (2 if n >= K.WIDE_PLAN_ENTRIES else 0)
 
@@ -379,13 +379,13 @@ class GqaMoeEngine:
         fmt = getattr(self.W, "expert_format", "bf16")
         if fmt != "bf16" and hasattr(self.moe, "forward_stored"):
             # experts served in their stored form (E4M3 block-scaled / MXFP4 / NVFP4): same exchange, quantised GEMMs
-            few = fmt == "fp8" and T <= K.W8_ROWS and not self.fixed_kv_split
-            self.launches += 3 if few else 6
+            self.launches += self.FEW_ROW_LAUNCHES if fmt == "fp8" and self.moe.skinny_fp8(ws.x[:T], L.w_gate, L.w_down) else 6
             return self.moe.forward_stored(fmt, ws.x[:T], logits, kw, L.w_gate, L.w_up, L.w_down, ws.h[:T], shared=shared, residual=ws.h[:T],
                                            norm_w=next_norm, eps=cfg.rms_eps, x_out=ws.x[:T] if next_norm is not None else None)
         self.moe.forward(ws.x[:T], logits, kw, L.w_gate, L.w_up, L.w_down, ws.h[:T], shared=shared, residual=ws.h[:T],
                          norm_w=next_norm, eps=cfg.rms_eps, x_out=ws.x[:T] if next_norm is not None else None)
-        self.launches += self._exchange_launches(T)             # plan(+dispatch), fc1, fc2, combine
+        few = isinstance(self.moe, LocalExchange) and self.moe.skinny(ws.x[:T], L.w_gate, L.w_down)
+        self.launches += self.FEW_ROW_LAUNCHES if few else self._exchange_launches(T)             # plan(+dispatch), fc1, fc2, combine
         return next_norm is not None
 
     # ---- whole step -------------------------------------------------------------------------------

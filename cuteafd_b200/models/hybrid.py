@@ -883,7 +883,7 @@ class HybridEngine:
                               swap=True if r.outputs % 4 else None)
             self.launches += 2
         moe.experts(h, logits, kw, L.w_gate, L.w_up, L.w_down)
-        self.launches += 4
+        self.launches += 2 if moe.skinny(h, L.w_gate, L.w_down) else 4
         return w, idx, r.experts, h
 
     # ---- whole step -------------------------------------------------------------------------------------------------

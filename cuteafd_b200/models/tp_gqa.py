@@ -149,7 +149,7 @@ class TpGqaMoeEngine(GqaMoeEngine):
         if self.pre_moe is not None:
             self.pre_moe(i)
         self.moe.forward(x, logits, dict(self.route_kw, bias=L.router_bias), L.w_gate, L.w_up, L.w_down, y, shared=shared)
-        self.launches += 6
+        self.launches += 5 if hasattr(self.moe, "skinny") and self.moe.skinny(x, L.w_gate, L.w_down) else 6
         return y
 
     def forward(self, b: Batch) -> torch.Tensor:

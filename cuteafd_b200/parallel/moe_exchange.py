@@ -325,6 +325,12 @@ class LocalExchange:
         return (0 < T and x.stride(0) == x.shape[1] and K.moe_skinny_ok(T * self.geo.top_k, T, w_gate, x)
                 and K.moe_skinny_ok(T * self.geo.top_k, T, w_down, x))
 
+    def skinny_fp8(self, x: torch.Tensor, w_gate: tuple, w_down: tuple) -> bool:
+        """The same for E4M3 experts given as (values, scales)."""
+        T = x.shape[0]
+        return (0 < T and x.stride(0) == x.shape[1] and K.moe_skinny_w8_ok(T * self.geo.top_k, T, w_gate[0], x)
+                and K.moe_skinny_w8_ok(T * self.geo.top_k, T, w_down[0], x))
+
     def _run_skinny(self, x: torch.Tensor, logits: torch.Tensor | None, route_kw: dict, w_gate: torch.Tensor, w_up: torch.Tensor,
                     w_down: torch.Tensor) -> None:
         T, k = x.shape[0], self.geo.top_k
@@ -378,8 +384,7 @@ class LocalExchange:
         each grouped GEMM."""
         T = x.shape[0]
         g = self.geo
-        if (tile_rows is None and wire is None and 0 < T and x.stride(0) == x.shape[1] and K.moe_skinny_w8_ok(T * g.top_k, T, w_gate[0], x)
-                and K.moe_skinny_w8_ok(T * g.top_k, T, w_down[0], x)):
+        if tile_rows is None and wire is None and self.skinny_fp8(x, w_gate, w_down):
             # a few rows: bf16 rows against the stored bytes, no plan, no slab and nothing quantised
             idx = self.att.idx[:T]
             if logits is not None:

@@ -502,3 +502,27 @@ def test_step_staging_is_not_overwritten_before_its_copy_ran():
     b.tokens[0][:] = 99
     torch.cuda.synchronize()
     assert [int(t[0]) for t in seen] == [1, 2, 3, 4] and all(bool((t == t[0]).all()) for t in seen)
+
+
+def test_launches_of_a_step_are_counted_by_the_form_that_it_took(monkeypatch):
+    """Experts whose width is no whole number of 64-element groups keep plan and dispatch at every step size, and are counted so."""
+    from cuteafd_b200.models.gqa_moe import GqaMoeEngine, GqaMoeWeights, KvCache
+    from cuteafd_b200.ops import kernels as K
+    from cuteafd_b200.runtime.generate import Generator
+    from cuteafd_b200.runtime.paged import PagePool
+    device, calls = torch.device("cuda", 0), []
+    for name in ("moe_plan", "moe_dispatch", "grouped_linear", "moe_skinny", "moe_combine"):
+        monkeypatch.setattr(K, name, lambda *a, _f=getattr(K, name), _n=name, **kw: (calls.append(_n), _f(*a, **kw))[1])
+    counted = []
+    for ffn in (128, 96):
+        cfg = small_cfg().replace(expert_ffn=ffn)
+        eng = GqaMoeEngine(cfg, GqaMoeWeights.random_init(cfg, device, seed=0), KvCache(cfg, 16, device), max_tokens=64, max_seqs=4)
+        gen = Generator(eng, PagePool(16), max_pages_per_seq=4, max_seqs=4, prefill_chunk=64, use_graphs=False)
+        seqs = [gen.table.new() for _ in range(2)]
+        last = [gen.prefill(s, list(range(20 + i))) for i, s in enumerate(seqs)]
+        calls.clear()
+        before = eng.launches
+        gen.decode(seqs, last)
+        assert ("moe_skinny" in calls, "moe_plan" in calls) == (ffn == 128, ffn == 96)
+        counted.append(eng.launches - before - len(calls))
+    assert counted[0] == counted[1]
