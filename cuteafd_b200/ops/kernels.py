@@ -382,8 +382,17 @@ def moe_skinny(x: torch.Tensor, row_div: int, w: torch.Tensor, w_up: torch.Tenso
     [E, N / 128, K / 128]: the weights are E4M3.  ``early``: the kernel launched last on this stream writes neither the weights nor ``idx``."""
     E, N, Kd = w.shape
     T, k = idx.shape
-    assert x.stride(1) == 1 and x.stride(0) == Kd and out.stride(1) == 1 and idx.is_contiguous() and w.is_contiguous()
-    assert scale is None or (scale.is_contiguous() and scale.dtype == torch.float32 and scale.shape == (E, N // 128, Kd // 128))
+    assert x.dtype == out.dtype == torch.bfloat16 and x.shape[1] == Kd and x.stride(1) == 1 and x.stride(0) == Kd
+    assert x.shape[0] * row_div >= T * k and out.shape[0] >= T * k and out.shape[1] >= N and out.stride(1) == 1
+    assert idx.dtype == torch.int32 and idx.is_contiguous()
+    for m, sc in ((w, scale), (w_up, scale_up)):
+        if m is None:
+            assert sc is None
+            continue
+        assert m.shape == w.shape and m.is_contiguous() and m.dtype == (torch.bfloat16 if scale is None else torch.float8_e4m3fn)
+        assert (sc is None) == (scale is None)
+        assert sc is None or (sc.is_contiguous() and sc.dtype == torch.float32 and sc.shape == (E, N // 128, Kd // 128))
+    assert expert_count is None or (expert_count.dtype == torch.int32 and expert_count.is_contiguous() and expert_count.numel() >= E)
     _n.check(_n.cuda_lib().cafd_moe_skinny(x.data_ptr(), row_div, w.data_ptr(), _ptr(w_up), _ptr(scale), _ptr(scale_up), idx.data_ptr(), T * k, T,
                                            E, Kd, N, out.data_ptr(), out.stride(0), _ptr(expert_count), int(early), num_sms(), _stream()),
              "moe_skinny")
@@ -393,7 +402,17 @@ def linear_w8(x: torch.Tensor, w: torch.Tensor, ws: torch.Tensor, out: torch.Ten
               ws_up: torch.Tensor | None = None, residual: torch.Tensor | None = None, resident: bool = False) -> torch.Tensor:
     """y = x @ dequant(w, ws).T for at most ``W8_ROWS`` bf16 rows and E4M3 weights [N, K] with scales [N / 128, K / 128]."""
     T, Kd = x.shape
-    assert x.is_contiguous() and x.dtype == torch.bfloat16 and w.is_contiguous() and ws.is_contiguous() and w.shape[1] == Kd
+    N = w.shape[0]
+    assert x.is_contiguous() and x.dtype == out.dtype == torch.bfloat16 and w.shape[1] == Kd
+    assert out.shape[0] >= T and out.shape[1] >= N and out.stride(1) == 1
+    assert residual is None or (residual.dtype == torch.bfloat16 and residual.shape[0] >= T and residual.shape[1] >= N and residual.stride(1) == 1
+                                 and (T == 1 or residual.stride(0) == out.stride(0)))
+    for m, sc in ((w, ws), (w_up, ws_up)):
+        if m is None:
+            assert sc is None
+            continue
+        assert m.shape == w.shape and m.is_contiguous() and m.dtype == torch.float8_e4m3fn
+        assert sc.is_contiguous() and sc.dtype == torch.float32 and sc.shape == (N // 128, Kd // 128)
     _n.check(_n.cuda_lib().cafd_linear_w8(x.data_ptr(), T, w.data_ptr(), _ptr(w_up), ws.data_ptr(), _ptr(ws_up), Kd, w.shape[0], out.data_ptr(),
                                           out.stride(0), _ptr(residual), int(resident), num_sms(), _stream()), "linear_w8")
     return out

@@ -106,3 +106,28 @@ def test_rotation_shares_angles_once_there_are_warps_enough():
         for heads in (3, 6, 10, 40, 112):
             T = -(-12 * sms // -(-heads // 8))
             assert per(1, heads, sms) == per(T - 1, heads, sms) == 1 and per(T, heads, sms) == per(1 << 20, heads, sms) == 8
+
+
+def test_few_row_operands_are_checked_before_their_addresses_are_used():
+    """Shapes, types and layouts that the kernel doesn't look at are refused by the wrappers; nothing here reaches a device."""
+    from cuteafd_b200.ops import kernels as K
+    bf, f8 = torch.bfloat16, torch.float8_e4m3fn
+    E, N, Kd, T, k = 4, 128, 256, 3, 2
+
+    def t(*shape, dtype=bf):
+        return torch.zeros(*shape, dtype=dtype)
+    ok = dict(x=t(T, Kd), row_div=k, w=t(E, N, Kd), w_up=t(E, N, Kd), idx=t(T, k, dtype=torch.int32), out=t(T * k, N))
+    f8s = dict(ok, w=t(E, N, Kd, dtype=f8), w_up=t(E, N, Kd, dtype=f8), scale=t(E, 1, 2, dtype=torch.float32), scale_up=t(E, 1, 2, dtype=torch.float32))
+    for base, bad in ((ok, dict(idx=t(T, k, dtype=torch.int64))), (ok, dict(w_up=t(E, N, Kd // 2))), (ok, dict(w_up=t(E, N, Kd, dtype=f8))), (ok, dict(w_up=t(E, Kd, N).mT)),
+                      (ok, dict(out=t(T * k - 1, N))), (ok, dict(out=t(T * k, N, dtype=torch.float32))), (ok, dict(out=t(T * k, N - 1))), (ok, dict(x=t(T - 1, Kd))),
+                      (ok, dict(x=t(T, Kd, dtype=torch.float16))), (ok, dict(x=t(T, 2 * Kd)[:, ::2])), (ok, dict(w=t(E, N, Kd, dtype=f8))), (ok, dict(scale_up=t(E, 1, 2, dtype=torch.float32))),
+                      (ok, dict(expert_count=t(E - 1, dtype=torch.int32))), (ok, dict(expert_count=t(E, dtype=torch.int64))), (f8s, dict(scale_up=None)),
+                      (f8s, dict(scale_up=t(E, 2, 1, dtype=torch.float32))), (f8s, dict(scale_up=t(E, 1, 2))), (f8s, dict(scale=t(E, 1, 1, dtype=torch.float32))), (f8s, dict(w_up=t(E, N, Kd)))):
+        with pytest.raises(AssertionError):
+            K.moe_skinny(**{**base, **bad})
+    lin = dict(x=t(T, Kd), w=t(N, Kd, dtype=f8), ws=t(1, 2, dtype=torch.float32), out=t(T, N), w_up=t(N, Kd, dtype=f8), ws_up=t(1, 2, dtype=torch.float32), residual=t(T, N))
+    for bad in (dict(ws=t(2, 1, dtype=torch.float32)), dict(ws=t(1, 2)), dict(w=t(N, Kd)), dict(w_up=t(N, Kd)), dict(w_up=t(N // 2, Kd, dtype=f8)), dict(ws_up=None),
+                dict(ws_up=t(1, 1, dtype=torch.float32)), dict(w_up=None), dict(out=t(T, N, dtype=torch.float32)), dict(out=t(T - 1, N)), dict(residual=t(T, N, dtype=torch.float32)),
+                dict(residual=t(T, 2 * N)[:, :N]), dict(x=t(T, Kd // 2))):
+        with pytest.raises((AssertionError, AttributeError)):
+            K.linear_w8(**{**lin, **bad})
