@@ -73,7 +73,7 @@ def test_sample_row_errors_and_accept_prefix():
     assert list(zip(acc.tolist(), bonus.tolist())) == want
 
 
-@pytest.mark.parametrize("V", [1, 7, 8, 1023, 8 * 1024 + 5, 131071, 8 * 48 * 1024 + 11])
+@pytest.mark.parametrize("V", [1, 7, 8, 1023, 8 * 1024 + 5, 131071, 262147, 8 * 48 * 1024 - 3, 8 * 48 * 1024 + 11])
 @pytest.mark.parametrize("shape", ["peaked", "flat", "ties"])
 def test_sample_rows_over_vocabularies(V, shape):
     """Slices that are empty, ragged, in shared memory and too long for it; tokens above the line that fit the sorted list (peaked) and

@@ -12,7 +12,7 @@ def _close(got, want, scale):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * scale).all()
 
 
-@pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 25, 32])
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 16, 17, 24, 25, 32])
 @pytest.mark.parametrize("N,K", [(1, 64), (17, 768), (40, 1024), (24, 1088), (5120, 2048), (2048, 4096), (37, 7168)])
 def test_dense_rows(T, N, K):
     from cuteafd_b200.ops import kernels as k
@@ -23,14 +23,15 @@ def test_dense_rows(T, N, K):
     a = x.double() @ w.double().T
     scale = K ** 0.5
     _close(k.linear(x, w, out_f32=True), a, scale)
-    for resident in (False, True):
-        h = torch.randn(T, N, device=DEV, generator=g).to(torch.bfloat16)
-        want = a + h.double()
-        out = torch.full((T, N + 8), 7.0, dtype=torch.bfloat16, device=DEV)[:, :N] if not resident else h
-        if resident:                              # in place, as the engines add to the residual stream
-            _close(k.linear(x, w, out=out, residual=h, resident=True), want, scale)
-        else:
-            _close(k.linear(x, w, out=out), a, scale)
+    # in rows of their own pitch, the columns between left alone
+    full, hs = torch.full((T, N + 8), 7.0, dtype=torch.bfloat16, device=DEV), torch.randn(T, N + 8, device=DEV, generator=g).to(torch.bfloat16)[:, :N]
+    _close(k.linear(x, w, out=full[:, :N]), a, scale)
+    assert (full[:, N:] == 7.0).all()
+    _close(k.linear(x, w, out=full[:, :N], residual=hs), a + hs.double(), scale)
+    assert (full[:, N:] == 7.0).all()
+    h = torch.randn(T, N, device=DEV, generator=g).to(torch.bfloat16)
+    want = a + h.double()                         # in place, as the engines add to the residual stream
+    _close(k.linear(x, w, out=h, residual=h, resident=True), want, scale)
     xs = x / scale
     b = xs.double() @ up.double().T
     c = xs.double() @ w.double().T
@@ -142,19 +143,29 @@ def test_e4m3_rows(T, N, K):
     _close(k.linear_w8(x, q, s, torch.empty_like(h), w_up=qu, ws_up=su), torch.nn.functional.silu(a) * b, 1.0 + a.abs() + b.abs())
 
 
-@pytest.mark.parametrize("T,top_k,E,I,H", [(1, 8, 256, 256, 384), (8, 8, 256, 128, 2304), (3, 2, 4, 384, 128)])
-def test_e4m3_experts_of_a_step(T, top_k, E, I, H):
+@pytest.mark.parametrize("T,top_k,E,I,H,spread", [(1, 8, 256, 256, 384, "random"), (8, 8, 256, 128, 2304, "random"), (3, 2, 4, 384, 128, "random"),
+                                                  (8, 8, 5, 128, 384, "same"), (8, 4, 6, 256, 256, "outside")])
+def test_e4m3_experts_of_a_step(T, top_k, E, I, H, spread):
+    """Spread routes, more routes on one expert than a column tile holds, and routes outside the stored ids."""
     from cuteafd_b200.ops import kernels as k
     g = torch.Generator(device=DEV).manual_seed(T + E)
     x = (torch.randn(T, H, device=DEV, generator=g) * H ** -0.5).to(torch.bfloat16)
     (qg, sg, gate), (qu, su, up), (qd, sd, down) = _e4m3((E, I, H), g), _e4m3((E, I, H), g), _e4m3((E, H, I), g)
-    idx = torch.rand(T, E, device=DEV, generator=g).topk(top_k).indices.to(torch.int32).contiguous()
+    if spread == "same":
+        idx = torch.full((T, top_k), 3, device=DEV)
+        idx[1, 2] = 4
+    else:
+        idx = torch.rand(T, E + (2 if spread == "outside" else 0), device=DEV, generator=g).topk(top_k).indices
+    idx = idx.to(torch.int32).contiguous()
     torch.cuda.synchronize()
-    hbuf, out = torch.empty(T * top_k, I, dtype=torch.bfloat16, device=DEV), torch.empty(T * top_k, H, dtype=torch.bfloat16, device=DEV)
+    hbuf, out = (torch.full((T * top_k, n), 3.0, dtype=torch.bfloat16, device=DEV) for n in (I, H))
     assert k.moe_skinny_w8_ok(T * top_k, T, qg, x) and k.moe_skinny_w8_ok(T * top_k, T, qd, x)
     k.moe_skinny(x, top_k, qg, qu, idx, hbuf, scale=sg, scale_up=su)
     k.moe_skinny(hbuf, 1, qd, None, idx, out, scale=sd, early=True)
     for e, ex in enumerate(idx.flatten().tolist()):
+        if ex >= E:
+            assert (hbuf[e] == 3.0).all() and (out[e] == 3.0).all()
+            continue
         c, b = gate[ex] @ x[e // top_k].double(), up[ex] @ x[e // top_k].double()
         _close(hbuf[e], torch.nn.functional.silu(c) * b, 1.0 + c.abs() + b.abs())
         _close(out[e], down[ex] @ hbuf[e].double(), I ** 0.5 * float(hbuf[e].abs().max()))
