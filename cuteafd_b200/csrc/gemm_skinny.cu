@@ -14,8 +14,8 @@
 //   * the experts read the tokens' rows where they are and write (token, slot) rows: every block sorts the step's routes (at most 256)
 //     by expert for itself, which takes the plan and dispatch launches out of a decode step.
 // Measured (in a chain with an RMSNorm, graph): 5120 x 2048 at 1 / 8 / 16 rows 5.9 / 6.4 / 8.0 us (tcgen05: 11.2 / 11.5 / 11.9), 2048 x 4096
-// 6.8 / 7.2 / 11.4 us (11.0 / 11.5 / 11.9); experts of 128 x (768, 2048), top-8, with combine, at 1 / 4 / 8 / 12 rows 24 / 60 / 93 / 140 us
-// (with plan and dispatch on tcgen05: 48 / 91 / 121 / 145).  Beyond that the activations' fragments, read once per 16 weight rows,
+// 6.8 / 7.2 / 11.4 us (11.0 / 11.5 / 11.9); experts of 128 x (768, 2048), top-8 over random routes, with combine, at 1 / 4 / 8 / 12 rows 28 / 58 / 90 /
+// 131 us (with plan and dispatch on tcgen05: 48 / 96 / 136 / 155).  Beyond that the activations' fragments, read once per 16 weight rows,
 // fill the L1 pipe and the tcgen05 kernel is the faster one.
 // E4M3 weights (128 x 128 block scales) are expanded to f16 in registers and meet the bf16 rows as f16, exactly over the range that matters
 // (sk_rows_f16): nothing is quantised, the error of the rows' E4M3 form is gone (logits of the DeepSeek-V3 geometry 1.2e-2 -> 8.7e-3 off

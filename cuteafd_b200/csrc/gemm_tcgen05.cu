@@ -571,7 +571,8 @@ static int launch(const cafd_gemm_args* a, cudaStream_t stream) {
 // Feature width of a dense product's 128-row tiles with tokens on the M side.  A chat-sized prompt's projection has few 128 x 256 tiles, and a
 // tile's K range is one block's serial chain: narrower tiles put more SMs to work (the sums of an element don't depend on the width), but
 // a narrow tile takes more than half a wide one's time, so they pay only while all of them run at once.  512 rows, 2048 x 4096: 32 tiles of
-// 256 50 us, 128 of 64 30 us; 777 rows: 56 of 256 47 us, 112 of 128 37 us; a router's 128 x 2048 at 777 rows 16 -> 13 us.  Where the
+// 256 50 us behind attention and 32 behind a norm, 128 of 64 30 and 29 us; 777 rows: 56 of 256 47 and 33 us, 112 of 128 37 and 31; a
+// router's 128 x 2048 at 777 rows 16 -> 13 us.  Where the
 // narrow ones take a second wave they lose: 640 rows, 2048 x 4096: 40 of 256 32 us, 160 of 64 49 us; 300 rows, 4096 x 14336: 48 of 256
 // 92 us, 192 of 64 160 us.
 extern "C" int cafd_gemm_prompt_tile(int rows, int features, int num_sms) {

@@ -380,8 +380,8 @@ class LocalExchange:
                     tile_rows: int | None = None, wire: bool | None = None, norm_w: torch.Tensor | None = None, eps: float = 0.0,
                     x_out: torch.Tensor | None = None) -> torch.Tensor:
         """Same exchange with E4M3 experts: each ``w_*`` is (values [E, N, K] e4m3, scales [E, N/128, K/128]).
-        Decode-sized steps quantise the rows 1x128 inside the dispatch (``wire``); otherwise on the expert side before
-        each grouped GEMM."""
+        A few rows meet the stored bytes as they are (``skinny_fp8``); decode-sized steps quantise the rows 1x128 inside the
+        dispatch (``wire``); otherwise on the expert side before each grouped GEMM."""
         T = x.shape[0]
         g = self.geo
         if tile_rows is None and wire is None and self.skinny_fp8(x, w_gate, w_down):
