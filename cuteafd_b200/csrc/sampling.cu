@@ -13,7 +13,7 @@
 // One cluster of one to eight blocks per row, each with its share of the vocabulary in shared memory as
 // order-preserving 32-bit keys.  What bounds the kernel is the number of dependent passes, not the
 // 0.6 MB a row is read once: with one block per row, walking the row from L2 in every pass, eight
-// rows of 151936 took 371 us and 32 rows of 129280 666 us, now 32 and 44 us.  One histogram over
+// rows of 151936 took 371 us and 32 rows of 129280 666 us, now 27 and 35 us.  One histogram over
 // (maximum - value) in steps of 1/8 says how far down the first filter can reach; the tokens above
 // that line, a few hundred for the settings that chats use, are gathered into one block, sorted,
 // and all filters and the draw are prefix sums over the sorted list.  When more than 2048 tokens
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   pdl_wait();
   pdl_trigger();
   __shared__ SampleShared sh;
-  extern __shared__ uint32_t sm_keys[];
+  extern __shared__ __align__(16) uint32_t sm_keys[];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = static_cast<int>(cluster.block_rank());
   const int out_row = blockIdx.x / kC;
@@ -279,8 +279,52 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
                          !(rp.min_p >= 0.f && rp.min_p <= 1.0f) || V <= 0;
   // ---- pass A: validation, max, lowest-id argmax; the logits stay in shared memory ---------------------
   float best = -INFINITY; int bi = 0x7fffffff; int cnt = 0, bad = 0;
-  constexpr int kAhead = 8;                       // loads in flight per thread (one after the other: 256 greedy rows of 262144 604 us, now 213)
-  for (int j0 = tid; j0 < n; j0 += kAhead * kSampleThreads) {
+  const bool greedy = rp.temperature < kGreedyEps || rp.top_k == 1, keep = in_smem && !greedy;
+  auto take = [&](int i, float v, bool allowed) {
+    const bool finite = isfinite(v);
+    cnt += allowed;
+    bad |= allowed && !finite;
+    if (allowed && finite && (v > best || (v == best && i < bi))) { best = v; bi = i; }
+  };
+  int from = 0;
+  if ((reinterpret_cast<uintptr_t>(x + id0) & 15u) == 0) {
+    // Sixteen logits in flight per thread, four to a load: a slice starts at a multiple of four tokens, so four share a mask word.  Where
+    // a slice leaves an SM one block, its loads in flight are the pass's rate: 256 greedy rows of 262144 tokens 209 us with eight 4-byte
+    // loads, 148 with these, of 151936 90 and 76 (one block per row and four blocks per SM: 145 and 90).  Eight vector loads: 142 and 134,
+    // their registers cost the second block where there is one.
+    constexpr int kAhead = 4;
+    const int n4 = n / 4;
+    const uint4* x4 = reinterpret_cast<const uint4*>(x + id0);
+    for (int c0 = tid; c0 < n4; c0 += kAhead * kSampleThreads) {
+      uint4 v[kAhead];
+      uint32_t in[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int c = c0 + q * kSampleThreads;
+        in[q] = c < n4 ? 0xfu : 0u;
+        v[q] = c < n4 ? __ldcg(x4 + c) : uint4{0u, 0u, 0u, 0u};
+      }
+      if (mask) {
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+          const int i = id0 + 4 * (c0 + q * kSampleThreads);
+          if (in[q]) in[q] = (__ldcg(mask + (i >> 5)) >> (i & 31)) & 0xfu;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int c = c0 + q * kSampleThreads, i = id0 + 4 * c;
+        if (keep && c < n4) reinterpret_cast<uint4*>(sm_keys)[c] = v[q];
+        take(i, __uint_as_float(v[q].x), in[q] & 1u);
+        take(i + 1, __uint_as_float(v[q].y), (in[q] >> 1) & 1u);
+        take(i + 2, __uint_as_float(v[q].z), (in[q] >> 2) & 1u);
+        take(i + 3, __uint_as_float(v[q].w), (in[q] >> 3) & 1u);
+      }
+    }
+    from = 4 * n4;
+  }
+  constexpr int kAhead = 8;                       // rows of another alignment, and a row's last tokens
+  for (int j0 = from + tid; j0 < n; j0 += kAhead * kSampleThreads) {
     float v[kAhead];
     bool in[kAhead];
 #pragma unroll
@@ -298,12 +342,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     }
 #pragma unroll
     for (int q = 0; q < kAhead; ++q) {
-      const int j = j0 + q * kSampleThreads, i = id0 + j;
-      if (in_smem && j < n) sm_keys[j] = __float_as_uint(v[q]);
-      const bool finite = isfinite(v[q]);
-      cnt += in[q];
-      bad |= in[q] && !finite;
-      if (in[q] && finite && (v[q] > best || (v[q] == best && i < bi))) { best = v[q]; bi = i; }
+      const int j = j0 + q * kSampleThreads;
+      if (keep && j < n) sm_keys[j] = __float_as_uint(v[q]);
+      take(id0 + j, v[q], in[q]);
     }
   }
   for (int o = 16; o; o >>= 1) {
@@ -338,7 +379,6 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   if (bad_param) status = kSampleBadParam;
   else if (cnt == 0) status = kSampleEmptyMask;
   else if (bad) status = kSampleNonFinite;
-  const bool greedy = rp.temperature < kGreedyEps || rp.top_k == 1;
   if (status != kSampleOk || greedy) {          // the same for all blocks of the row
     if (rank == 0 && tid == 0) { out_token[out_row] = status != kSampleOk ? -1 : bi; out_status[out_row] = status; }
     cluster.sync();                             // no block leaves while another reads its share
@@ -500,7 +540,8 @@ struct SampleCall {
 
 template <int kC>
 static int launch_sample(const SampleCall& c, cudaStream_t st) {
-  const int slice = c.V > 0 ? static_cast<int>((static_cast<long long>(c.V) + kC - 1) / kC) : 0;
+  // a slice starts at a multiple of four tokens
+  const int slice = c.V <= 0 ? 0 : kC == 1 ? c.V : static_cast<int>((static_cast<long long>(c.V) + 4 * kC - 1) / (4 * kC)) * 4;
   const size_t smem = slice <= kSampleSmemKeys ? static_cast<size_t>(slice) * 4 : 0;
   CAFD_CHECK_CUDA(cudaFuncSetAttribute(sample_rows_kernel<kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmemKeys * 4));
   cudaLaunchConfig_t cfg = {};
@@ -527,7 +568,7 @@ using namespace cafd;
 
 // Blocks per row: eight, and fewer for a batch that would not be resident at once (two blocks to an SM) as long as a slice's keys still
 // stay in shared memory beside another block's.  Clusters of a fixed eight, and one block that reads its row again in every pass, against
-// this, us: 256 greedy rows of 8192 41 / 16 / 11, of 32000 51 / 23 / 20; 256 rows of 8192, top-k 50 and top-p 0.95, 101 / 79 / 26.  Keys
+// this (first pass with four-byte loads), us: 256 greedy rows of 8192 41 / 16 / 11, of 32000 51 / 23 / 20; 256 rows of 8192, top-k 50 and top-p 0.95, 101 / 79 / 26.  Keys
 // that don't stay in shared memory cost more than the further waves: 256 rows of 151936, top-p 0.9, 296 us with eight blocks, 555 with one.
 extern "C" int cafd_sample_cluster(int n, int V, int num_sms) {
   int c = 8;

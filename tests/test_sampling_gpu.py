@@ -145,3 +145,31 @@ def test_zeros_of_both_signs_are_one_value(V):
     tok, st = (torch.full((40,), -7, dtype=torch.int32, device=dev) for _ in range(2))
     K.sample_rows(logits.to(dev), K.pack_sample_rows(params, positions).to(dev), tok, st)
     assert st.tolist() == status and tok.tolist() == want
+
+
+@pytest.mark.parametrize("n", [6, 300])
+@pytest.mark.parametrize("V,ld", [(3, 4), (2047, 2050), (2048, 2048), (2050, 2052), (16387, 16389), (16388, 16392)])
+@pytest.mark.parametrize("first", [0, 1])
+def test_sample_rows_of_any_alignment(n, V, ld, first):
+    """Rows that start on a 16-byte boundary and rows that don't, whole and broken groups of four tokens, with and without a mask."""
+    from cuteafd_b200.ops import kernels as K
+    from cuteafd_b200.runtime.sampling import SamplingParams, select_rows
+    dev = torch.device("cuda", 0)
+    kinds = [dict(), dict(temperature=0.7, top_k=50, top_p=0.95), dict(temperature=1.0, top_p=0.8)]
+    params = [SamplingParams(seed=i, **kinds[i % 3]) for i in range(n)]
+    g = torch.Generator().manual_seed(V + ld)
+    whole = torch.full((n * ld + 8,), float("nan"))                     # what lies between rows is nobody's token
+    on_host = whole[first:].as_strided((n, V), (ld, 1))
+    on_host.copy_((torch.randn(n, V, generator=g) * 128).round() / 64)
+    logits = whole.to(dev)[first:].as_strided((n, V), (ld, 1))
+    words = (V + 31) // 32
+    allowed = torch.rand(words * 32, generator=g) < 0.4
+    allowed[V - 1] = True
+    w = (allowed.view(words, 32).long() << torch.arange(32)).sum(1)
+    bits = torch.where(w >= 2 ** 31, w - 2 ** 32, w).to(torch.int32).to(dev)
+    tok, st = (torch.full((n,), -7, dtype=torch.int32, device=dev) for _ in range(2))
+    rows = K.pack_sample_rows(params, list(range(n)), mask_word0=[0 if i % 2 else None for i in range(n)]).to(dev)
+    K.sample_rows(logits, rows, tok, st, masks=bits)
+    some = list(range(0, n, 1 if n < 10 else 23))
+    want, status = select_rows(on_host[some].contiguous(), [params[i] for i in some], some, [allowed[:V] if i % 2 else None for i in some])
+    assert not st.any() and status == [0] * len(some) and tok[some].tolist() == want
