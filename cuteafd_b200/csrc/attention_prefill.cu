@@ -153,7 +153,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   pdl_wait();      // the page table, lengths and Q come from kernels earlier in the stream
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int seq = blockIdx.z;
   const int head = blockIdx.y;
   const int kvh = head / (p.Hq / p.Hkv);
@@ -260,69 +260,70 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = make_idesc(128, 128, 1, 1, 0, 0);
-      constexpr uint32_t idesc_pv = make_idesc(128, 128, 1, 1, 0, 1);   // B = V is MN-major
-      const uint32_t aQ = smem_u32(sQ), aP = smem_u32(sP);
-      bool ok = mbar_wait(&q_full, 0, p.status, kTimeoutFullBarrier);
-      auto issue_qk = [&](int u) -> bool {
-        const int j = u / kMaps, st = j & 1, sb = u & 1;
-        if ((kMaps == 1 || sb == 0) && !mbar_wait(&k_full[st], (j >> 1) & 1, p.status, kTimeoutFullBarrier)) return false;
-        if (!mbar_wait(&s_empty[sb], ((u >> 1) & 1) ^ 1, p.status, kTimeoutTmemEmpty)) return false;
-        tc_fence_after();
-        const uint32_t aK = smem_u32(sK + st * kTileB);
+    constexpr uint32_t idesc_qk = make_idesc(128, 128, 1, 1, 0, 0);
+    constexpr uint32_t idesc_pv = make_idesc(128, 128, 1, 1, 0, 1);   // B = V is MN-major
+    const uint64_t dQ = smem_desc_k_sw128(smem_u32(sQ)), dK = smem_desc_k_sw128(smem_u32(sK)), dP = smem_desc_k_sw128(smem_u32(sP));
+    const uint64_t dV = smem_desc_mn_sw128(smem_u32(sV), kHalfBytes);
+    bool ok = mbar_wait_warp(&q_full, 0, p.status, kTimeoutFullBarrier);
+    auto issue_qk = [&](int u) -> bool {
+      const int j = u / kMaps, st = j & 1, sb = u & 1;
+      if ((kMaps == 1 || sb == 0) && !mbar_wait_warp(&k_full[st], (j >> 1) & 1, p.status, kTimeoutFullBarrier)) return false;
+      if (!mbar_wait_warp(&s_empty[sb], ((u >> 1) & 1) ^ 1, p.status, kTimeoutTmemEmpty)) return false;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t k0 = dK + static_cast<uint64_t>(st * (kTileB >> 4));
+        const uint32_t d = tS + sb * 128;
         if (kMaps == 2) {
+          const uint64_t half = static_cast<uint64_t>(sb * (kHalfBytes >> 4));
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_f16(tS + sb * 128, smem_desc_k_sw128(aQ + sb * kHalfBytes + k4 * 32),
-                     smem_desc_k_sw128(aK + sb * kHalfBytes + k4 * 32), idesc_qk, k4 ? 1u : 0u);
+          for (int k4 = 0; k4 < 4; ++k4) umma_f16(d, dQ + half + k4 * 2, k0 + half + k4 * 2, idesc_qk, k4 ? 1u : 0u);
           if (sb == 1) umma_commit(&k_empty[st]);
-          umma_commit(&s_full[sb]);
-          return true;
+        } else {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4)
+              umma_f16(d, dQ + h * (kHalfBytes >> 4) + k4 * 2, k0 + h * (kHalfBytes >> 4) + k4 * 2, idesc_qk, (h | k4) ? 1u : 0u);
+          if (kRope) {
+            const uint64_t dQr = smem_desc_k_sw128(smem_u32(sQr)), dKr = smem_desc_k_sw128(smem_u32(sKr)) + static_cast<uint64_t>(st * (kHalfBytes >> 4));
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4) umma_f16(d, dQr + k4 * 2, dKr + k4 * 2, idesc_qk, 1u);
+          }
+          umma_commit(&k_empty[st]);
         }
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_f16(tS + st * 128, smem_desc_k_sw128(aQ + h * kHalfBytes + k4 * 32),
-                     smem_desc_k_sw128(aK + h * kHalfBytes + k4 * 32), idesc_qk, (h | k4) ? 1u : 0u);
-        if (kRope) {
-          const uint32_t aQr = smem_u32(sQr), aKr = smem_u32(sKr + st * kHalfBytes);
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_f16(tS + st * 128, smem_desc_k_sw128(aQr + k4 * 32), smem_desc_k_sw128(aKr + k4 * 32), idesc_qk, 1u);
-        }
-        umma_commit(&k_empty[st]);
-        umma_commit(&s_full[st]);
-        return true;
-      };
-      // Scores run two tiles ahead of P V: the softmax warps release a score buffer as soon as they have read it
-      // into registers, so S(j + 2) is computed while they work on tile j and S(j + 1) is already waiting.
-      // (The kRope variant has one V stage: its producer cannot load K(j + 2) before P V(j) has freed V, so there
-      // the scores stay one tile ahead.)
-      constexpr int kAhead = kVS == 2 ? 2 : 1;
-      if (ok) ok = issue_qk(0);
-      if (ok && kAhead == 2 && n_units > 1) ok = issue_qk(1);
-      for (int u = 0; ok && u < n_units; ++u) {
-        if (u + kAhead < n_units) { if (!issue_qk(u + kAhead)) { ok = false; break; } }
-        const int j = u / kMaps, pb = u % kPB;
-        if (!mbar_wait(&p_ready[pb], (u / kPB) & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
-        const int vs = kVS == 2 ? (j & 1) : 0;
-        const uint32_t vph = kVS == 2 ? ((j >> 1) & 1) : (j & 1);
-        if ((kMaps == 1 || pb == 0) && !mbar_wait(&v_full[vs], vph, p.status, kTimeoutFullBarrier)) { ok = false; break; }
-        tc_fence_after();
+        umma_commit(&s_full[sb]);
+      }
+      __syncwarp();
+      return true;
+    };
+    // Scores run two tiles ahead of P V: the softmax warps release a score buffer as soon as they have read it
+    // into registers, so S(j + 2) is computed while they work on tile j and S(j + 1) is already waiting.
+    // (The kRope variant has one V stage: its producer cannot load K(j + 2) before P V(j) has freed V, so there
+    // the scores stay one tile ahead.)
+    constexpr int kAhead = kVS == 2 ? 2 : 1;
+    if (ok) ok = issue_qk(0);
+    if (ok && kAhead == 2 && n_units > 1) ok = issue_qk(1);
+    for (int u = 0; ok && u < n_units; ++u) {
+      if (u + kAhead < n_units) { if (!issue_qk(u + kAhead)) { ok = false; break; } }
+      const int j = u / kMaps, pb = u % kPB;
+      if (!mbar_wait_warp(&p_ready[pb], (u / kPB) & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+      const int vs = kVS == 2 ? (j & 1) : 0;
+      const uint32_t vph = kVS == 2 ? ((j >> 1) & 1) : (j & 1);
+      if ((kMaps == 1 || pb == 0) && !mbar_wait_warp(&v_full[vs], vph, p.status, kTimeoutFullBarrier)) { ok = false; break; }
+      tc_fence_after();
+      if (elect_one()) {
         const uint32_t tOm = kMaps == 2 ? tO + pb * 128 : tO;
-        const uint32_t aV = smem_u32(sV + vs * kTileB);
+        const uint64_t p0 = dP + static_cast<uint64_t>(pb * (kTileB >> 4)), v0 = dV + static_cast<uint64_t>(vs * (kTileB >> 4));
 #pragma unroll
         for (int k8 = 0; k8 < 8; ++k8) {
           // A = P: atom (k8 / 4) of 64 kv columns, 32 bytes per K step inside it
           // B = V: 16 kv rows per step (2 KiB), two 64-wide d halves 16 KiB apart
-          umma_f16(tOm, smem_desc_k_sw128(aP + pb * kTileB + (k8 >> 2) * kHalfBytes + (k8 & 3) * 32),
-                   smem_desc_mn_sw128(aV + k8 * 2048, kHalfBytes), idesc_pv, (j | k8) ? 1u : 0u);
+          umma_f16(tOm, p0 + (((k8 >> 2) * kHalfBytes + (k8 & 3) * 32) >> 4), v0 + (k8 * 2048 >> 4), idesc_pv, (j | k8) ? 1u : 0u);
         }
         if (kMaps == 1 || pb == 1) umma_commit(&v_empty[vs]);
         umma_commit(&pv_done[pb]);
       }
+      __syncwarp();
     }
   } else {
     // Eight softmax warps: warps w and w + 4 share a TMEM lane quarter (32 query rows) and split the tile's 128

@@ -43,6 +43,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// A value that all lanes of the warp hold, told to the compiler.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -103,6 +106,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
       return false;
     }
   }
+}
+
+// The same by a whole warp, the answer alike in all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
 
 // ---- TMA ---------------------------------------------------------------------------------------
@@ -174,6 +182,10 @@ __device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// How the MMA warps issue: the whole warp walks the stages and elect_one() names the lane that issues and commits.  Descriptors and addresses
+// then stay in uniform registers.  Issued under `lane == 0`, each tcgen05.mma took some 100 cycles of moves into them, longer than a product
+// of 128 x 128 x 16 takes (64).
+
 // Arrive on an mbarrier when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))

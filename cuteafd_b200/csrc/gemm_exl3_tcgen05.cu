@@ -72,7 +72,7 @@ gemm_exl3_kernel(const __grid_constant__ CUtensorMap tm_x, const Exl3Dev p) {
   __shared__ uint64_t tfull_bar[2];
   __shared__ uint64_t tempty_bar[2];
   __shared__ uint32_t tmem_base_slot;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::kStages; ++s) { mbar_init(&full_bar[s], 1 + 128); mbar_init(&empty_bar[s], 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(&tfull_bar[s], 1); mbar_init(&tempty_bar[s], 128); }
@@ -108,30 +108,34 @@ gemm_exl3_kernel(const __grid_constant__ CUtensorMap tm_x, const Exl3Dev p) {
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(128, kBX, 0, 0);          // fp16 x fp16 -> fp32
-      int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+    constexpr uint32_t idesc = make_idesc(128, kBX, 0, 0);          // fp16 x fp16 -> fp32
+    const uint64_t wdesc = smem_desc_k_sw128(smem_u32(smem)), xdesc = smem_desc_k_sw128(smem_u32(smem) + kXWBytes);
+    int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + acc * kBX;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + acc * kBX;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes), sx = sw + kXWBytes;
+        if (elect_one()) {
+          const uint64_t sw = wdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
+          const uint64_t sx = xdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
 #pragma unroll
           for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4)
-              umma_f16(d0, smem_desc_k_sw128(sw + a * (kXRows * 128) + k4 * 32), smem_desc_k_sw128(sx + a * (kBX * 128) + k4 * 32),
-                       idesc, ((kb - kb0) | a | k4) ? 1u : 0u);
+              umma_f16(d0, sw + ((a * (kXRows * 128) + k4 * 32) >> 4), sx + ((a * (kBX * 128) + k4 * 32) >> 4), idesc,
+                       ((kb - kb0) | a | k4) ? 1u : 0u);
           umma_commit(&empty_bar[stage]);
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(&tfull_bar[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else if (warp >= 6) {
     // ------------------------------------------------------------------ trellis decoders

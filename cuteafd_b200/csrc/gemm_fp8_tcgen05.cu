@@ -91,7 +91,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant
   __shared__ int s_x_tiles;
   __shared__ int s_last_unit;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -163,39 +163,40 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(128, Cfg::kMmaN, 0, 0);    // E4M3 x E4M3 -> fp32
-      int stage = 0;
-      uint32_t phase = 0;
-      uint32_t it = 0;                 // K blocks issued by this CTA (selects the partial buffer)
-      bool ok = true;
-      for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x) {
-        const int split = unit % splits;
-        const int kb0 = split * nkb / splits, kb1 = (split + 1) * nkb / splits;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int pb = it & 1;
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
-          if (!mbar_wait(&pempty_bar[pb], ((it >> 1) & 1) ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
-          tc_fence_after();
+    constexpr uint32_t idesc = make_idesc(128, Cfg::kMmaN, 0, 0);    // E4M3 x E4M3 -> fp32
+    const uint64_t wdesc = smem_desc_k_sw128(smem_u32(smem)), xdesc = smem_desc_k_sw128(smem_u32(smem) + Cfg::kWTiles * Cfg::kWBytes);
+    int stage = 0;
+    uint32_t phase = 0;
+    uint32_t it = 0;                 // K blocks issued by this CTA (selects the partial buffer)
+    bool ok = true;
+    for (int unit = blockIdx.x; ok && unit < total_units; unit += gridDim.x) {
+      const int split = unit % splits;
+      const int kb0 = split * nkb / splits, kb1 = (split + 1) * nkb / splits;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int pb = it & 1;
+        if (!mbar_wait_warp(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
+        if (!mbar_wait_warp(&pempty_bar[pb], ((it >> 1) & 1) ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
           const uint32_t d0 = tmem_base + pb * Cfg::kAccCols;
-          const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t sx = sw + Cfg::kWTiles * Cfg::kWBytes;
+          const uint64_t sw = wdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
+          const uint64_t sx = xdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
 #pragma unroll
           for (int k4 = 0; k4 < kF8BK / kF8UmmaK; ++k4) {
-            const uint32_t koff = k4 * kF8UmmaK;
+            constexpr uint32_t kStep = kF8UmmaK >> 4;
             const uint32_t accum = k4 ? 1u : 0u;
             if (kSwap) {
-              umma_f8(d0, smem_desc_k_sw128(sw + koff), smem_desc_k_sw128(sx + koff), idesc, accum);
-              if (kDual)
-                umma_f8(d0 + kBX, smem_desc_k_sw128(sw + Cfg::kWBytes + koff), smem_desc_k_sw128(sx + koff), idesc, accum);
+              umma_f8(d0, sw + k4 * kStep, sx + k4 * kStep, idesc, accum);
+              if (kDual) umma_f8(d0 + kBX, sw + (Cfg::kWBytes >> 4) + k4 * kStep, sx + k4 * kStep, idesc, accum);
             } else {
-              umma_f8(d0, smem_desc_k_sw128(sx + koff), smem_desc_k_sw128(sw + koff), idesc, accum);
+              umma_f8(d0, sx + k4 * kStep, sw + k4 * kStep, idesc, accum);
             }
           }
           umma_commit(&empty_bar[stage]);
           umma_commit(&pfull_bar[pb]);
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else {

@@ -105,7 +105,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ C
   __shared__ int s_last_unit;
   __shared__ void* s_rs_out[8];
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -193,46 +193,46 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(Cfg::kMmaM, Cfg::kMmaN, 1, 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int unit = blockIdx.x; ok && unit < total_tiles; unit += gridDim.x) {
-        const int split = unit % splits;
-        const int kb0 = split * nkb / splits, kb1 = (split + 1) * nkb / splits;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+    constexpr uint32_t idesc = make_idesc(Cfg::kMmaM, Cfg::kMmaN, 1, 1);
+    const uint64_t wdesc = smem_desc_k_sw128(smem_u32(smem)), xdesc = smem_desc_k_sw128(smem_u32(smem) + Cfg::kWTiles * Cfg::kWBytes);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int unit = blockIdx.x; ok && unit < total_tiles; unit += gridDim.x) {
+      const int split = unit % splits;
+      const int kb0 = split * nkb / splits, kb1 = (split + 1) * nkb / splits;
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + acc * Cfg::kAccCols;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + acc * Cfg::kAccCols;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t sx = sw + Cfg::kWTiles * Cfg::kWBytes;
+        if (elect_one()) {
+          const uint64_t sw = wdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
+          const uint64_t sx = xdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
 #pragma unroll
           for (int k4 = 0; k4 < kBK / kUmmaK; ++k4) {
-            const uint32_t koff = k4 * kUmmaK * 2;
+            constexpr uint32_t kStep = kUmmaK * 2 >> 4;
             const uint32_t accum = ((kb - kb0) | k4) ? 1u : 0u;
             if (kSwap) {
               // A = weights (128 features), B = tokens (kBX)
-              umma_f16(d0, smem_desc_k_sw128(sw + koff), smem_desc_k_sw128(sx + koff), idesc, accum);
-              if (kDual)
-                umma_f16(d0 + kBX, smem_desc_k_sw128(sw + Cfg::kWBytes + koff), smem_desc_k_sw128(sx + koff), idesc,
-                         accum);
+              umma_f16(d0, sw + k4 * kStep, sx + k4 * kStep, idesc, accum);
+              if (kDual) umma_f16(d0 + kBX, sw + (Cfg::kWBytes >> 4) + k4 * kStep, sx + k4 * kStep, idesc, accum);
             } else {
               // A = tokens (128 rows), B = weights (kBW or 2*kBW rows, gate then up, contiguous)
-              umma_f16(d0, smem_desc_k_sw128(sx + koff), smem_desc_k_sw128(sw + koff), idesc, accum);
+              umma_f16(d0, sx + k4 * kStep, sw + k4 * kStep, idesc, accum);
             }
           }
           umma_commit(&empty_bar[stage]);
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+          if (kb == kb1 - 1) umma_commit(&tfull_bar[acc]);
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else {
     // ------------------------------------------------------------------ epilogue (4 warps)

@@ -95,7 +95,7 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
   __shared__ uint32_t tmem_base_slot;
   __shared__ int s_x_tiles;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -170,38 +170,40 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(128, kBX, 1, 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+    constexpr uint32_t idesc = make_idesc(128, kBX, 1, 1);
+    const uint64_t wdesc = smem_desc_k_sw128(smem_u32(smem)), xdesc = smem_desc_k_sw128(smem_u32(smem) + Cfg::kWTiles * kW4WBytes);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t d0 = tmem_base + acc * Cfg::kAccCols;
+      for (int kb = 0; kb < nkb; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d0 = tmem_base + acc * Cfg::kAccCols;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, kTimeoutFullBarrier)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes);
-          const uint32_t sx = sw + Cfg::kWTiles * kW4WBytes;
+        if (elect_one()) {
+          const uint64_t sw = wdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
+          const uint64_t sx = xdesc + static_cast<uint64_t>(stage * (Cfg::kStageBytes >> 4));
 #pragma unroll
           for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4) {
               const uint32_t accum = (kb | a | k4) ? 1u : 0u;
-              const uint32_t wo = a * (kW4Rows * 128) + k4 * 32, xo = a * (kBX * 128) + k4 * 32;
-              umma_f16(d0, smem_desc_k_sw128(sw + wo), smem_desc_k_sw128(sx + xo), idesc, accum);
-              if (kDual) umma_f16(d0 + kBX, smem_desc_k_sw128(sw + kW4WBytes + wo), smem_desc_k_sw128(sx + xo), idesc, accum);
+              const uint32_t wo = (a * (kW4Rows * 128) + k4 * 32) >> 4, xo = (a * (kBX * 128) + k4 * 32) >> 4;
+              umma_f16(d0, sw + wo, sx + xo, idesc, accum);
+              if (kDual) umma_f16(d0 + kBX, sw + (kW4WBytes >> 4) + wo, sx + xo, idesc, accum);
             }
           umma_commit(&empty_bar[stage]);
-          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+          if (kb == nkb - 1) umma_commit(&tfull_bar[acc]);
         }
-        if (!ok) break;
-        umma_commit(&tfull_bar[acc]);
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   } else if (warp == 10) {
     // ------------------------------------------------------------------ packed-weight TMA producer

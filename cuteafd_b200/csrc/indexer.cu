@@ -57,7 +57,7 @@ indexer_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   pdl_wait();
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int blk = blockIdx.x, split = blockIdx.y;
   const int seq = p.block_seq[blk], tok0 = p.block_tok0[blk];
   const int q0 = p.q_start[seq], q_len = p.q_start[seq + 1] - q0;
@@ -115,25 +115,27 @@ indexer_scores_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
       constexpr uint32_t idesc = make_idesc(128, kIdxN, 1, 1, 0, 0);
-      const uint32_t aQ = smem_u32(sQ);
-      bool ok = mbar_wait(&q_full, 0, p.status, kTimeoutFullBarrier);
+      const uint64_t dQ = smem_desc_k_sw128(smem_u32(sQ)), dK = smem_desc_k_sw128(smem_u32(sK));
+      bool ok = mbar_wait_warp(&q_full, 0, p.status, kTimeoutFullBarrier);
       for (int j = 0; ok && j < n_tiles; ++j) {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&k_full[st], ph, p.status, kTimeoutFullBarrier)) break;
-        if (!mbar_wait(&d_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty)) break;
+        if (!mbar_wait_warp(&k_full[st], ph, p.status, kTimeoutFullBarrier)) break;
+        if (!mbar_wait_warp(&d_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty)) break;
         tc_fence_after();
-        const uint32_t aK = smem_u32(sK + st * kIdxKBytes);
+        if (elect_one()) {
+          const uint64_t k0 = dK + static_cast<uint64_t>(st * (kIdxKBytes >> 4));
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+          for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_f16(tmem + st * kIdxN, smem_desc_k_sw128(aK + a * kIdxKv * 128 + k4 * 32),
-                     smem_desc_k_sw128(aQ + a * kIdxN * 128 + k4 * 32), idesc, (a | k4) ? 1u : 0u);
-        umma_commit(&k_empty[st]);
-        umma_commit(&d_full[st]);
+            for (int k4 = 0; k4 < 4; ++k4)
+              umma_f16(tmem + st * kIdxN, k0 + ((a * kIdxKv * 128 + k4 * 32) >> 4), dQ + ((a * kIdxN * 128 + k4 * 32) >> 4), idesc, (a | k4) ? 1u : 0u);
+          umma_commit(&k_empty[st]);
+          umma_commit(&d_full[st]);
+        }
+        __syncwarp();
       }
     }
   } else {

@@ -94,7 +94,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   pdl_wait();
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int blk = blockIdx.x, dh = blockIdx.y, split = blockIdx.z;
   const int seq = p.block_seq[blk];
   const int tok0 = p.block_tok0[blk];
@@ -213,27 +213,31 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0) {
       constexpr uint32_t idesc_qk = make_idesc(128, kKvTile, 1, 1, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc(128, kHalf, 1, 1, 0, 1);      // B = V is MN-major
-      const uint32_t aQ = smem_u32(sQ), aP = smem_u32(sP);
-      bool ok = mbar_wait(&q_full, 0, p.status, kTimeoutFullBarrier);
-      mla_trace(tr, 1, ok ? 1 : 2);
+      const uint64_t dQ = smem_desc_k_sw128(smem_u32(sQ)), dC = smem_desc_k_sw128(smem_u32(sC)), dP = smem_desc_k_noswz(smem_u32(sP), 128, 512);
+      const uint64_t dV = smem_desc_mn_sw128(smem_u32(sC) + dh * 4 * (kKvTile * 128), kKvTile * 128);
+      bool ok = mbar_wait_warp(&q_full, 0, p.status, kTimeoutFullBarrier);
+      if (lane == 0) mla_trace(tr, 1, ok ? 1 : 2);
       auto issue_qk = [&](int j) -> bool {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&c_full[st], ph, p.status, kTimeoutFullBarrier)) return false;
-        if (!mbar_wait(&s_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty)) return false;
+        if (!mbar_wait_warp(&c_full[st], ph, p.status, kTimeoutFullBarrier)) return false;
+        if (!mbar_wait_warp(&s_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty)) return false;
         tc_fence_after();
-        const uint32_t aC = smem_u32(sC + st * kKvBytes);
-#pragma unroll 1
-        for (int a = 0; a < kAtoms; ++a)
+        if (elect_one()) {
+          const uint64_t c0 = dC + static_cast<uint64_t>(st * (kKvBytes >> 4));
 #pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)
-            umma_f16(tS + st * 32, smem_desc_k_sw128(aQ + a * kMlaRows * 128 + k4 * 32),
-                     smem_desc_k_sw128(aC + a * kKvTile * 128 + k4 * 32), idesc_qk, (a | k4) ? 1u : 0u);
-        umma_commit(&s_full[st]);
-        mla_trace(tr, 1, 100 + j);
+          for (int a = 0; a < kAtoms; ++a)
+#pragma unroll
+            for (int k4 = 0; k4 < 4; ++k4)
+              umma_f16(tS + st * 32, dQ + ((a * kMlaRows * 128 + k4 * 32) >> 4), c0 + ((a * kKvTile * 128 + k4 * 32) >> 4), idesc_qk,
+                       (a | k4) ? 1u : 0u);
+          umma_commit(&s_full[st]);
+          mla_trace(tr, 1, 100 + j);
+        }
+        __syncwarp();
         return true;
       };
       if (ok) ok = issue_qk(0);
@@ -243,24 +247,26 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int nst = (j + 1) & 1;
         const uint32_t nph = ((j + 1) >> 1) & 1;
         bool next_done = j + 1 >= n_tiles;
-        if (!next_done && mbar_try_wait(&c_full[nst], nph) && mbar_try_wait(&s_empty[nst], nph ^ 1)) {
+        if (!next_done && __all_sync(0xffffffffu, mbar_try_wait(&c_full[nst], nph) && mbar_try_wait(&s_empty[nst], nph ^ 1))) {
           if (!issue_qk(j + 1)) { ok = false; break; }
           next_done = true;
         }
         const int st = j & 1;
-        if (!mbar_wait(&p_ready, j & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+        if (!mbar_wait_warp(&p_ready, j & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t aV = smem_u32(sC + st * kKvBytes) + dh * 4 * (kKvTile * 128);
+        if (elect_one()) {
+          const uint64_t v0 = dV + static_cast<uint64_t>(st * (kKvBytes >> 4));
 #pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          // A = P rows, K cores ks*2 and ks*2+1 (128 bytes apart), 8-row groups 512 bytes apart
-          // B = V: 16 kv rows per step (2 KiB), 64-column blocks 4 KiB apart, 8-row groups 1 KiB apart
-          umma_f16(tO, smem_desc_k_noswz(aP + ks * 256, 128, 512), smem_desc_mn_sw128(aV + ks * 2048, kKvTile * 128),
-                   idesc_pv, (j | ks) ? 1u : 0u);
+          for (int ks = 0; ks < 2; ++ks) {
+            // A = P rows, K cores ks*2 and ks*2+1 (128 bytes apart), 8-row groups 512 bytes apart
+            // B = V: 16 kv rows per step (2 KiB), 64-column blocks 4 KiB apart, 8-row groups 1 KiB apart
+            umma_f16(tO, dP + (ks * 256 >> 4), v0 + (ks * 2048 >> 4), idesc_pv, (j | ks) ? 1u : 0u);
+          }
+          umma_commit(&c_empty[st]);
+          umma_commit(&pv_done);
+          mla_trace(tr, 1, 10000 + j);
         }
-        umma_commit(&c_empty[st]);
-        umma_commit(&pv_done);
-        mla_trace(tr, 1, 10000 + j);
+        __syncwarp();
         if (!next_done && !issue_qk(j + 1)) { ok = false; break; }
       }
     }
