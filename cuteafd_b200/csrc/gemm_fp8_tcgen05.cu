@@ -319,7 +319,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant
           bool row_ok = p.tile_row0 ? true : (row < p.x_rows);
           if (p.row_dst && row_ok) { dst = p.row_dst[row]; row_ok = dst >= 0; }
           if (row_ok && f_ok) {
-            float val = kDual ? silu(acc[j]) * acc[kBX + j] : acc[j];
+            float val = kDual ? silu_tile(acc[j]) * acc[kBX + j] : acc[j];
             const size_t off = static_cast<size_t>(dst) * p.ldo + f;
             if (p.residual) val += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.residual)[off]);
             reinterpret_cast<__nv_bfloat16*>(p.out)[off] = __float2bfloat16(val);
@@ -339,7 +339,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant
           for (int j = 0; j < kOutCols; j += 8) {
             float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = kDual ? silu(acc[j + e]) * acc[kBW + j + e] : acc[j + e];
+            for (int e = 0; e < 8; ++e) v[e] = kDual ? silu_tile(acc[j + e]) * acc[kBW + j + e] : acc[j + e];
             if (f0 + j + 8 <= p.n_features) {
               if (rs) {
                 const uint4 q = *reinterpret_cast<const uint4*>(rs + j);

@@ -311,7 +311,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ C
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 const float g = __uint_as_float(r[j]), uj = __uint_as_float(u[j]);
-                v[j] = (kClip ? clipped_glu(g, uj, p.glu) : silu(g) * uj) * scale;
+                v[j] = (kClip ? clipped_glu(g, uj, p.glu) : silu_tile(g) * uj) * scale;
               }
             } else {
               tmem_ld_wait();
@@ -409,7 +409,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ C
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = !kDual ? g[j] : kClip ? clipped_glu(g[j], u[j], p.glu) : silu(g[j]) * u[j];
+            for (int j = 0; j < 16; ++j) v[j] = !kDual ? g[j] : kClip ? clipped_glu(g[j], u[j], p.glu) : silu_tile(g[j]) * u[j];
           } else {
             uint32_t r[16];
             tmem_ld_32x16(t0 + c0, r);
@@ -419,7 +419,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ C
               tmem_ld_wait();
 #pragma unroll
               for (int j = 0; j < 16; ++j)
-                v[j] = kClip ? clipped_glu(__uint_as_float(r[j]), __uint_as_float(u[j]), p.glu) : silu(__uint_as_float(r[j])) * __uint_as_float(u[j]);
+                v[j] = kClip ? clipped_glu(__uint_as_float(r[j]), __uint_as_float(u[j]), p.glu) : silu_tile(__uint_as_float(r[j])) * __uint_as_float(u[j]);
             } else {
               tmem_ld_wait();
 #pragma unroll

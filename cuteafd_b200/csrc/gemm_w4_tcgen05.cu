@@ -360,7 +360,7 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
           tmem_ld_32x16(t0 + kBX + c0, uu);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = silu(__uint_as_float(rr[j]) * g0) * (__uint_as_float(uu[j]) * g1);
+          for (int j = 0; j < 16; ++j) v[j] = silu_tile(__uint_as_float(rr[j]) * g0) * (__uint_as_float(uu[j]) * g1);
         } else {
           tmem_ld_wait();
 #pragma unroll
