@@ -41,7 +41,7 @@ MAX_RANKS = 8
 WAIT_LIMIT_SETTERS = ("cafd_gemm_set_wait_limit_ns", "cafd_moe_set_wait_limit_ns", "cafd_attn_set_wait_limit_ns",
                       "cafd_gemm_fp8_set_wait_limit_ns", "cafd_tp_set_wait_limit_ns", "cafd_mla_set_wait_limit_ns",
                       "cafd_indexer_set_wait_limit_ns", "cafd_gemm_w4_set_wait_limit_ns", "cafd_gemm_exl3_set_wait_limit_ns",
-                      "cafd_decode_step_set_wait_limit_ns")
+                      "cafd_decode_step_set_wait_limit_ns", "cafd_gemm_w8_set_wait_limit_ns")
 
 
 BOUNDS_UNITS = ("cafd_moe", "cafd_tp")        # translation units with checked peer-store sites
@@ -195,6 +195,7 @@ def cuda_lib():
         P, I, F = C.c_void_p, C.c_int, C.c_float
         _sig(lib, "cafd_gemm", [C.POINTER(GemmArgs), P])
         _sig(lib, "cafd_gemm_fp8", [C.POINTER(GemmArgs), P])
+        _sig(lib, "cafd_gemm_w8", [C.POINTER(GemmArgs), P])
         _sig(lib, "cafd_quant_rows_fp8", [P, P, P, I, I, I, P])
         for n in WAIT_LIMIT_SETTERS:
             _sig(lib, n, [C.c_ulonglong])

@@ -83,6 +83,9 @@ int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream);
 int cafd_gemm_prompt_tile(int rows, int features, int num_sms);
 int cafd_gemm_few_rows(const cafd_gemm_args* a);     // whether cafd_gemm runs it on the few-row kernel
 
+int cafd_gemm_w8(const cafd_gemm_args* a, cafd_stream_t stream);       // grouped: E4M3 weights, bf16 rows (gemm_w8_tcgen05.cu)
+int cafd_gemm_w8_set_wait_limit_ns(unsigned long long ns);
+
 // ---- greedy selection ----------------------------------------------------------------------------
 // out[t] = argmax over logits[t, 0:V] (row pitch ld, fp32); ties go to the lowest index and NaN is
 // never selected.  `scratch` holds 2 * T * cafd_argmax_slices() 4-byte words, owned by the caller.

@@ -379,7 +379,8 @@ class GqaMoeEngine:
         fmt = getattr(self.W, "expert_format", "bf16")
         if fmt != "bf16" and hasattr(self.moe, "forward_stored"):
             # experts served in their stored form (E4M3 block-scaled / MXFP4 / NVFP4): same exchange, quantised GEMMs
-            self.launches += self.FEW_ROW_LAUNCHES if fmt == "fp8" and self.moe.skinny_fp8(ws.x[:T], L.w_gate, L.w_down) else 6
+            few = fmt == "fp8" and self.moe.skinny_fp8(ws.x[:T], L.w_gate, L.w_down)
+            self.launches += self.FEW_ROW_LAUNCHES if few else self._exchange_launches(T) if fmt == "fp8" else 6
             return self.moe.forward_stored(fmt, ws.x[:T], logits, kw, L.w_gate, L.w_up, L.w_down, ws.h[:T], shared=shared, residual=ws.h[:T],
                                            norm_w=next_norm, eps=cfg.rms_eps, x_out=ws.x[:T] if next_norm is not None else None)
         self.moe.forward(ws.x[:T], logits, kw, L.w_gate, L.w_up, L.w_down, ws.h[:T], shared=shared, residual=ws.h[:T],

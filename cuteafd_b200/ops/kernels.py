@@ -1192,6 +1192,33 @@ def grouped_linear_fp8(xq: torch.Tensor, xs: torch.Tensor, wq: torch.Tensor, ws:
     _n.check(_n.cuda_lib().cafd_gemm_fp8(C.byref(a), _stream()), "cafd_gemm_fp8(grouped)")
 
 
+def grouped_linear_w8(x: torch.Tensor, w: tuple, out: torch.Tensor, tile_expert: torch.Tensor, tile_row0: torch.Tensor,
+                      num_tiles: torch.Tensor, max_tiles: int, tile_rows: int, *, w_up: tuple | None = None, row_dst: torch.Tensor | None = None,
+                      wait_flag: int | None = None, epoch: torch.Tensor | None = None, signal_flag: int | None = None,
+                      done_counter: torch.Tensor | None = None, out_ptr: int | None = None, ldo: int | None = None) -> None:
+    """Expert-grouped product of a bf16 slab with E4M3 experts, expanded on their way to the tensor cores: ``w`` (and ``w_up``: SwiGLU
+    pair) = (values [E, N, K], scales [E, N / 128, K / 128]); segments padded to ``tile_rows`` of 32, 64 or 128."""
+    E, N, Kd = w[0].shape
+    assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape[1] == Kd and N % 128 == 0 and Kd % 128 == 0
+    for q, s in (w, w_up) if w_up else (w,):
+        assert q.shape == (E, N, Kd) and s.shape == (E, N // 128, Kd // 128) and q.is_contiguous() and s.is_contiguous() and s.dtype == torch.float32
+    a = _n.GemmArgs()
+    a.w0, a.w1, a.x = w[0].data_ptr(), (w_up[0].data_ptr() if w_up else None), x.data_ptr()
+    a.w_scale, a.w_scale1 = w[1].data_ptr(), (w_up[1].data_ptr() if w_up else None)
+    a.out = out_ptr if out_ptr is not None else out.data_ptr()
+    a.row_dst = _ptr(row_dst)
+    a.tile_expert, a.tile_row0, a.num_x_tiles = tile_expert.data_ptr(), tile_row0.data_ptr(), num_tiles.data_ptr()
+    a.wait_flag, a.epoch = wait_flag, _ptr(epoch)
+    a.signal_flag, a.done_counter = signal_flag, _ptr(done_counter)
+    a.status = status_word(x.device).data_ptr()
+    a.w_rows_total, a.x_rows_total = E * N, x.shape[0]
+    a.k, a.n_features, a.x_rows = Kd, N, x.shape[0]
+    a.ldo = ldo if ldo is not None else out.stride(0)
+    a.w_rows_per_expert, a.max_x_tiles = N, max_tiles
+    a.swap, a.dual, a.bx, a.num_sms = 1, int(w_up is not None), tile_rows, num_sms()
+    _n.check(_n.cuda_lib().cafd_gemm_w8(C.byref(a), _stream()), "cafd_gemm_w8")
+
+
 # ---- 4-bit weights (MXFP4 / NVFP4) --------------------------------------------------------------------------
 W4_FORMATS = {"mxfp4": 2, "nvfp4": 3}
 

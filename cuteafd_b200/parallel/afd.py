@@ -399,6 +399,7 @@ class ExpertWorker:
         layers = range(min(self.n_main, self.n_layers)) if mtp == 0 else [self.n_main + mtp - 1]
         for l in layers:
             wg, wu, wd = self.weights[l]
+            expanded = False                     # this layer's E4M3 experts stand in memory as bf16
             for a in active:
                 T = counts[a]
                 for w, (t0, t1) in enumerate(g.waves(T)):
@@ -409,8 +410,8 @@ class ExpertWorker:
                     tile_rows = plan_tile_rows(fmt, t1 - t0, g.top_k, g.num_experts, g.expert_ffn, g.hidden)
                     if fmt == "fp8":                 # E4M3 values + 128x128 block scales
                         rows = min(side.geo.max_rows, (t1 - t0) * g.top_k + (hi - lo) * tile_rows)
-                        side.run_fp8(wg, wu, wd, tile_rows, rows, dslot, self.epochs[a], combine_ptr, flag, wait=True,
-                                     reuse_dequant=(w > 0 or a != active[0]), wire=wire_fp8_ok(side.geo, tile_rows))
+                        expanded |= side.run_fp8(wg, wu, wd, tile_rows, rows, dslot, self.epochs[a], combine_ptr, flag, wait=True,
+                                                 reuse_dequant=expanded, wire=wire_fp8_ok(side.geo, tile_rows))
                     elif fmt in ("mxfp4", "nvfp4"):
                         side.run_w4_any(fmt, wg, wu, wd, tile_rows, dslot, self.epochs[a], combine_ptr, flag,
                                         reuse_dequant=(w > 0 or a != active[0]))

@@ -54,9 +54,9 @@ def pick_tile_rows(T: int, top_k: int, num_experts: int, ffn: int = 0, hidden: i
 def plan_tile_rows(fmt: str, T: int, top_k: int, num_experts: int, ffn: int = 0, hidden: int = 0) -> int:
     """Row tile of a step's expert segments for experts stored as ``fmt``.  Both halves of an exchange derive it from
     the same arguments: the planner pads every expert's segment to it and the grouped GEMMs walk the tiles with it.
-    Quantised experts read their packed weights directly up to 64-row tiles; 128-row tiles mean the layer's experts are
-    expanded to bf16 first, which only pays once every expert sees at least 64 rows on average.  32-bit experts ("fp32") are
-    multiplied in blocks of 64 rows, padding included."""
+    Quantised experts read their packed weights directly up to 64-row tiles; 128-row tiles mean bf16 rows against experts that are
+    expanded, 4-bit ones in memory, E4M3 ones in the tile (``w8_expands``), from 64 rows for every expert on average on.  32-bit experts
+    ("fp32") are multiplied in blocks of 64 rows, padding included."""
     if fmt == "bf16":
         return pick_tile_rows(T, top_k, num_experts, ffn, hidden)
     avg = T * top_k / max(1, num_experts)
@@ -64,9 +64,39 @@ def plan_tile_rows(fmt: str, T: int, top_k: int, num_experts: int, ffn: int = 0,
     return 128 if t == 64 and avg >= (48 if fmt == "fp32" else 64) else t
 
 
+def w8_tile_rows(T: int, top_k: int, num_experts: int) -> int:
+    """Row tile of E4M3 experts that meet bf16 rows (``K.grouped_linear_w8``): the narrowest that holds nearly every segment, since another
+    tile reads and expands its expert again while columns of padding only cost products.  Whole exchange of 256 experts of (2048, 7168), top-8,
+    us on tiles of 32 / 64 / 128 rows (quantised rows before, expanded in memory from a mean of 64 on):
+
+    =====  ====================  ======
+    mean   32 / 64 / 128         before
+    =====  ====================  ======
+    1      1329 / 1413 / 1669    1338
+    8      2229 / 2417 / 3141    2677
+    16     2306 / 2532 / 3090    2796
+    31     3130 / 2403 / 2740    5558
+    47     4382 / 2424 / 3136    5094
+    64     5150 / 3482 / 3218    6532
+    94     6101 / 4690 / 3150    11193
+    256    16302 / 11516 / 7420  14538
+    =====  ====================  ======
+
+    32 experts of (768, 2048): 91 to 94 on tiles of 32 or 64 up to a mean of 32 (112 to 126 before)."""
+    avg = T * top_k / max(1, num_experts)
+    return 32 if avg <= 20 else 64 if avg <= 48 else 128
+
+
+def w8_expands(entries: int, num_experts: int) -> bool:
+    """Whether a step is so large that a layer's E4M3 experts are expanded in memory once instead of in every row tile: from a mean of 512
+    rows on.  Expanded in the tile / in memory at a mean of 384, 512, 768, 1024 rows: 64 experts of (2048, 7168) 2443 / 4534, 3145 / 4709,
+    4489 / 5848, 6335 / 6907 us; 32 of (768, 2048) 231 / 271, 284 / 311, 405 / 396, 490 / 464."""
+    return entries > 512 * num_experts
+
+
 def wire_fp8_ok(geo: "ExchangeGeometry", tile_rows: int) -> bool:
     """Whether a step's rows travel as E4M3 + per-128 scales: the block-scaled expert GEMM consumes them as they are
-    (decode-sized tiles); prefill-sized steps expand the experts to bf16 and want bf16 rows.  Both sides of the
+    (decode-sized tiles); prefill-sized steps expand the experts and want bf16 rows.  Both sides of the
     exchange call this with the same arguments."""
     return tile_rows < 128 and geo.hidden % 128 == 0
 
@@ -161,16 +191,28 @@ class ExpertSide:
                          signal_flag=combine_flag_ptr, done_counter=self.done[0:1] if combine_flag_ptr else None)
 
 
+    def run_w8(self, w_gate, w_up, w_down, tile_rows: int, layer: int, epoch: torch.Tensor, combine_ptr: int, combine_flag_ptr: int | None,
+               wait: bool) -> None:
+        """E4M3 experts against bf16 rows (slab and fc1 output), expanded inside the grouped GEMMs."""
+        g = self.geo
+        K.grouped_linear_w8(self.slab, w_gate, self.hbuf, self.tile_expert, self.tile_row0, self.num_tiles, g.max_tiles, tile_rows, w_up=w_up,
+                            epoch=epoch, wait_flag=(self.flags.data_ptr() + 4 * layer) if wait else None)
+        K.grouped_linear_w8(self.hbuf, w_down, self.hbuf, self.tile_expert, self.tile_row0, self.num_tiles, g.max_tiles, tile_rows,
+                            row_dst=self.row_dst, out_ptr=combine_ptr, ldo=g.hidden, epoch=epoch, signal_flag=combine_flag_ptr,
+                            done_counter=self.done[0:1] if combine_flag_ptr else None)
+
     def run_fp8(self, w_gate, w_up, w_down, tile_rows: int, rows: int, layer: int, epoch: torch.Tensor, combine_ptr: int,
-                combine_flag_ptr: int | None, wait: bool, reuse_dequant: bool = False, wire: bool = False) -> None:
+                combine_flag_ptr: int | None, wait: bool, reuse_dequant: bool = False, wire: bool = False) -> bool:
         """E4M3 experts: ``w_*`` = (values [E, N, K], scales [E, N/128, K/128]).  Received rows and the
         fc1 output are quantised 1x128 here, next to the GEMMs that consume them; with ``wire`` the rows arrived
-        quantised by the dispatch (``wire_q`` / ``wire_s``) and fc1 itself waits for the dispatch flag."""
+        quantised by the dispatch (``wire_q`` / ``wire_s``) and fc1 itself waits for the dispatch flag.  ``rows`` bounds the slab rows, padding
+        included.  Returns whether the layer's experts now stand expanded in memory, which is what ``reuse_dequant`` tells a later call."""
         g = self.geo
+        if tile_rows == 128 and not reuse_dequant and not w8_expands(rows - w_gate[0].shape[0] * tile_rows, g.num_experts):
+            self.run_w8(w_gate, w_up, w_down, tile_rows, layer, epoch, combine_ptr, combine_flag_ptr, wait)
+            return False
         if tile_rows == 128:
-            # Prefill-sized step: the block-scaled kernel folds scales in its epilogue warps and falls behind the bf16
-            # kernel at large row counts, so this layer's experts are expanded to bf16 (one layer's worth of scratch,
-            # reused by every layer) and the bf16 grouped GEMMs run instead.
+            # A very large step: one layer's worth of scratch, reused by every layer
             dq = ExpertSide._dq_scratch.get(w_gate[0].device)
             if dq is None or dq[0].shape != w_gate[0].shape:
                 dq = tuple(torch.empty(w[0].shape, dtype=torch.bfloat16, device=w[0].device) for w in (w_gate, w_up, w_down))
@@ -180,7 +222,7 @@ class ExpertSide:
                 for w, o in zip((w_gate, w_up, w_down), self._dq):
                     K.fp8_dequant_block128(w[0], w[1], o)
             self.run(self._dq[0], self._dq[1], self._dq[2], tile_rows, layer, epoch, combine_ptr, combine_flag_ptr, wait)
-            return
+            return True
         if not hasattr(self, "slab_q"):
             dev = self.slab.device
             self.slab_q = torch.zeros(g.max_rows, g.hidden, dtype=torch.float8_e4m3fn, device=dev)
@@ -203,6 +245,7 @@ class ExpertSide:
                              self.num_tiles, g.max_tiles, tile_rows, row_dst=self.row_dst, out_ptr=combine_ptr, ldo=g.hidden,
                              epoch=epoch, signal_flag=combine_flag_ptr,
                              done_counter=self.done[0:1] if combine_flag_ptr else None)
+        return False
 
     def run_w4(self, fmt: str, w_gate, w_up, w_down, tile_rows: int, layer: int, epoch: torch.Tensor, combine_ptr: int,
                combine_flag_ptr: int | None, wait: bool) -> None:
@@ -380,8 +423,9 @@ class LocalExchange:
                     tile_rows: int | None = None, wire: bool | None = None, norm_w: torch.Tensor | None = None, eps: float = 0.0,
                     x_out: torch.Tensor | None = None) -> torch.Tensor:
         """Same exchange with E4M3 experts: each ``w_*`` is (values [E, N, K] e4m3, scales [E, N/128, K/128]).
-        A few rows meet the stored bytes as they are (``skinny_fp8``); decode-sized steps quantise the rows 1x128 inside the
-        dispatch (``wire``); otherwise on the expert side before each grouped GEMM."""
+        A few rows meet the stored bytes as they are (``skinny_fp8``), larger steps expand them in the tile or, very large ones, in memory.  A
+        ``tile_rows`` below 128 or a ``wire`` of one's own asks for rows quantised 1x128, inside the dispatch (``wire``) or on the expert side
+        before each grouped GEMM."""
         T = x.shape[0]
         g = self.geo
         if tile_rows is None and wire is None and self.skinny_fp8(x, w_gate, w_down):
@@ -392,14 +436,19 @@ class LocalExchange:
             K.moe_skinny(x, g.top_k, w_gate[0], w_up[0], idx, self.exp.hbuf, scale=w_gate[1], scale_up=w_up[1], expert_count=self.att.expert_count)
             K.moe_skinny(self.exp.hbuf, 1, w_down[0], None, idx, self.att.combine, scale=w_down[1], early=True)
             return self.att.combine_into(out, T, 0, self.epoch, shared=shared, residual=residual, wait=False, norm_w=norm_w, eps=eps, x_out=x_out)
-        tile_rows = tile_rows or plan_tile_rows("fp8", T, g.top_k, g.num_experts)
+        e = self.exp
+        own = tile_rows is None and wire is None
+        tile_rows = tile_rows or (w8_tile_rows(T, g.top_k, g.num_experts) if own else plan_tile_rows("fp8", T, g.top_k, g.num_experts))
+        if own or tile_rows == 128:
+            self.att.dispatch(x, logits, route_kw, tile_rows, 0, self.epoch)
+            if tile_rows == 128:
+                e.run_fp8(w_gate, w_up, w_down, tile_rows, T * g.top_k + g.num_experts * tile_rows, 0, self.epoch, self.att.combine.data_ptr(), None,
+                          wait=False)
+            else:
+                e.run_w8(w_gate, w_up, w_down, tile_rows, 0, self.epoch, self.att.combine.data_ptr(), None, wait=False)
+            return self.att.combine_into(out, T, 0, self.epoch, shared=shared, residual=residual, wait=False, norm_w=norm_w, eps=eps, x_out=x_out)
         wire = wire_fp8_ok(g, tile_rows) if wire is None else wire
         self.att.dispatch(x, logits, route_kw, tile_rows, 0, self.epoch, wire_fp8=wire)
-        e = self.exp
-        if tile_rows == 128:
-            # prefill-sized step: expand this layer's experts to bf16 once and take the bf16 grouped GEMMs
-            e.run_fp8(w_gate, w_up, w_down, tile_rows, 0, 0, self.epoch, self.att.combine.data_ptr(), None, wait=False)
-            return self.att.combine_into(out, T, 0, self.epoch, shared=shared, residual=residual, wait=False, norm_w=norm_w, eps=eps, x_out=x_out)
         rows = min(g.max_rows, T * g.top_k + g.num_experts * tile_rows)
         if not hasattr(e, "slab_q"):
             dev = e.slab.device

@@ -131,3 +131,9 @@ def test_few_row_operands_are_checked_before_their_addresses_are_used():
                 dict(residual=t(T, 2 * N)[:, :N]), dict(x=t(T, Kd // 2))):
         with pytest.raises((AssertionError, AttributeError)):
             K.linear_w8(**{**lin, **bad})
+
+
+def test_w8_rules():
+    from cuteafd_b200.parallel.moe_exchange import w8_expands, w8_tile_rows
+    assert [w8_tile_rows(n * 32, 8, 256) for n in (1, 20, 21, 48, 49, 300)] == [32, 32, 64, 64, 128, 128]
+    assert not w8_expands(512 * 16, 16) and w8_expands(512 * 16 + 1, 16)
