@@ -41,7 +41,7 @@ MAX_RANKS = 8
 WAIT_LIMIT_SETTERS = ("cafd_gemm_set_wait_limit_ns", "cafd_moe_set_wait_limit_ns", "cafd_attn_set_wait_limit_ns",
                       "cafd_gemm_fp8_set_wait_limit_ns", "cafd_tp_set_wait_limit_ns", "cafd_mla_set_wait_limit_ns",
                       "cafd_indexer_set_wait_limit_ns", "cafd_gemm_w4_set_wait_limit_ns", "cafd_gemm_exl3_set_wait_limit_ns",
-                      "cafd_decode_step_set_wait_limit_ns", "cafd_gemm_w8_set_wait_limit_ns")
+                      "cafd_decode_step_set_wait_limit_ns", "cafd_gemm_w8_set_wait_limit_ns", "cafd_attn_pair_set_wait_limit_ns")
 
 
 BOUNDS_UNITS = ("cafd_moe", "cafd_tp")        # translation units with checked peer-store sites
@@ -237,7 +237,9 @@ def cuda_lib():
         _sig(lib, "cafd_attn_merge", [P, P, P, I, I, I, I, I, P])
         _sig(lib, "cafd_set_fixed_kv_split", [I])
         _sig(lib, "cafd_fixed_kv_split", [])
-        _sig(lib, "cafd_attn_prefill", [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, I, I, F, F, F, P, P, I, F, P, P])
+        _sig(lib, "cafd_attn_prefill", [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, I, I, F, F, F, P, P, I, F, P, P, I, P])
+        _sig(lib, "cafd_attn_prefill_splits", [I, I, I, I, I, I])
+        _sig(lib, "cafd_attn_prefill_scratch_floats", [I, I, I], C.c_longlong)
         _sig(lib, "cafd_mla_scratch_floats", [I, I], C.c_longlong)
         _sig(lib, "cafd_mla_attention", [P, P, P, P, P, P, P, P, P, P, C.c_longlong, I, I, I, I, I, I, F, P, I, I, P])
         _sig(lib, "cafd_indexer_scores", [P, P, P, I, F, P, P, P, P, P, P, P, C.c_longlong, I, I, I, I, I, I, P])

@@ -1,6 +1,7 @@
 // Causal GQA prefill attention over the paged KV cache on tcgen05 tensor cores (head_dim 128).
 //
-// One CTA computes a 128-row query tile of one head.  S = Q K^T and O += P V both run as
+// For what the two-tile kernel (attention_pair.cu) does not take: two score maps, capped scores, turned outputs, an odd number of heads to a kv
+// head, expanded MLA of one row tile.  One CTA computes a 128-row query tile of one head.  S = Q K^T and O += P V both run as
 // tcgen05.mma with accumulators in TMEM; K/V pages arrive by TMA straight from the page pool
 // (a 4-D tensor map indexed by page id), so chunked prefill and prefix-cache hits need no
 // gather.  Warp roles:
@@ -39,45 +40,13 @@
 #include "cafd_api.h"
 #include "common.cuh"
 #include "host_tma.h"
+#include "prefill.cuh"
 
 namespace cafd {
 
-constexpr int kHD = 128;          // head dim
-constexpr int kBQ = 128;          // query rows per CTA
-constexpr int kBKV = 128;         // kv tokens per tile (two 64-token pages)
-constexpr int kPageTok = 64;
-constexpr int kHalfBytes = 128 * 128;   // 128 rows x 64 bf16 (one swizzle atom wide) = 16 KiB
-constexpr int kTileB = 2 * kHalfBytes;  // 32 KiB: a [128 x 128] bf16 tile as two 64-wide halves
 constexpr int kPrefillThreads = 320;   // TMA warp, MMA warp, 8 softmax warps
 constexpr int kPrefillSmem = 7 * kTileB + 1024;   // Q, K x2, V x2, P x2
 constexpr int kPrefillSmemRope = 5 * kTileB + 3 * kHalfBytes + 1024;   // Q, Qr, (K, Kr) x2, V x1, P
-
-struct PrefillDev {
-  const int* page_table;   // [seqs, max_pages]
-  const int* seq_lens;     // kv length per sequence (including this chunk)
-  const int* q_start;      // [seqs + 1] row offsets into q/out
-  __nv_bfloat16* out;      // [total_q, Hq, 128]
-  uint32_t* status;
-  int max_pages;
-  int Hq, Hkv;
-  float scale_log2;
-  int window;              // sliding window: a query at position t sees keys (t - window, t]; 0 = all earlier keys
-  int keep;                // with a window: and the keys [0, keep)
-  int ldo;                 // elements from row to row of out
-  // kMaps == 2 only
-  float lambda, out_scale, eps;
-  // kMaps == 1 only
-  const float* sink;              // [Hq] or null
-  const __nv_bfloat16* gate;      // row t, head h: gate[t * gate_ld + h]; or null
-  int gate_ld;
-  const float2* v_table;          // [rows, 64] cos, sin; or null
-  float cap_in, cap_log2;         // scale / cap, cap * log2(e); scale_log2 is then 1.  These two and v_table: kTurn only
-  // kRope only
-  const int* kv_tmp_start; // [seqs] first row of the sequence in the expansion buffers (multiple of 64)
-  int q_head_stride;       // elements between heads in the nope query matrix (192 for [T, heads * 192])
-  int qr_head_stride;      // elements between heads in the rope query matrix (576 for the absorbed-query buffer)
-  int qr_col0;             // first rope column inside a head of that matrix (512)
-};
 
 // tanh(x) / x as a polynomial in x^2, fitted over |x| <= kTanhRange by least squares at Chebyshev nodes: within 2e-8
 constexpr float kTanhRange = 0.75f;
@@ -555,16 +524,41 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
 using namespace cafd;
 
+// Whether cafd_attn_prefill hands a step to the two-tile kernel: plain heads in pairs that share a kv head.
+static bool attn_prefill_paired(int Hq, int Hkv, int maps, bool turn) { return maps == 1 && !turn && (Hq / Hkv) % 2 == 0; }
+
+// Shares of a step's keys on the two-tile kernel, where its blocks leave SMs idle: as many as make the rounds of the blocks over the SMs, counted in
+// key tiles (1.9 us), shortest.  A block costs about two tiles on top of its own, the merge three and each share's rows their bytes written
+// and read.  512 rows of 32 heads behind 16384 tokens in 1 / 2 / 3 / 4 / 7 shares: 248 / 150 / 204 / 168 / 216 us (the counts here: 255 / 145 /
+// 190 / 152 / 190); 65 rows in 1 / 8: 239 / 50; 300 rows behind 1000 in 1 / 3: 28 / 45.
+extern "C" int cafd_attn_prefill_splits(int num_seqs, int max_q_len, int kv_tokens, int Hq, int Hkv, int num_sms) {
+  if (num_seqs < 1 || max_q_len < 1 || kv_tokens < 1 || Hkv < 1 || Hq % Hkv || (Hq / Hkv) % 2 || fixed_kv_split_tokens() > 0) return 1;
+  const long long sms = num_sms > 0 ? num_sms : 148, blocks = static_cast<long long>((max_q_len + kBQ - 1) / kBQ) * (Hq / 2) * num_seqs;
+  const long long tiles = (static_cast<long long>(kv_tokens) + kBKV - 1) / kBKV;
+  if (blocks >= sms) return 1;
+  int best = 1;
+  double least = static_cast<double>(tiles + 2);
+  for (int s = 2; s <= kPairSplits && tiles / s >= kPairShareTiles; ++s) {
+    const double cost = static_cast<double>((blocks * s + sms - 1) / sms * ((tiles + s - 1) / s + 2)) + 3 + 1.4e-4 * s * num_seqs * max_q_len * Hq;
+    if (cost < least) { least = cost; best = s; }
+  }
+  return best;
+}
+extern "C" long long cafd_attn_prefill_scratch_floats(int total_q, int Hq, int splits) {
+  return splits > 1 ? static_cast<long long>(splits) * total_q * Hq * (kHD + 2) : 0;
+}
+
 // q [total_q, Hq, 128] bf16 (two maps: [total_q, Hq, 2, 64]); out rows of ldo elements, head h's 128 values at column 128 h;
 // caches [num_pages, Hkv, 64, 128] bf16 (page 0 all zero); page_table [num_seqs, max_pages]; seq_lens [num_seqs];
 // q_start [num_seqs + 1]; max_q_len = longest chunk (grid sizing).  maps 1: lambda and eps are unused.
 // sink [Hq], gate rows (gate_ld elements apart), v_table [total_q, 64] (cos, sin of the output's rotation back) and cap (0 = none): one
-// map only.
+// map only.  splits > 1 (cafd_attn_prefill_splits): `scratch` holds cafd_attn_prefill_scratch_floats.
 extern "C" int cafd_attn_prefill(const void* q, const void* k_cache, const void* v_cache, const int* page_table,
                                  const int* seq_lens, const int* q_start, void* out, uint32_t* status, int total_q,
                                  int num_seqs, int max_q_len, int num_pages, int max_pages, int Hq, int Hkv, int D,
                                  float scale, int window, int keep, int ldo, int maps, float lambda, float out_scale, float eps,
-                                 const float* sink, const void* gate, int gate_ld, float cap, const void* v_table, cafd_stream_t s) {
+                                 const float* sink, const void* gate, int gate_ld, float cap, const void* v_table, float* scratch, int splits,
+                                 cafd_stream_t s) {
   if (num_seqs <= 0 || total_q <= 0) return 0;
   if (D != kHD || Hq % Hkv || window < 0 || keep < 0 || maps < 1 || maps > 2 || ldo < Hq * kHD || ldo % 8) return -10;
   if ((maps == 2 && (sink || gate || v_table || cap > 0.f)) || (gate && gate_ld < Hq)) return -10;
@@ -584,6 +578,7 @@ extern "C" int cafd_attn_prefill(const void* q, const void* k_cache, const void*
   rc = make_tmap_nd(&tv, v_cache, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, dims, strides, box, true);
   if (rc) return rc;
   PrefillDev p{};
+  p.total_q = total_q;
   p.page_table = page_table;
   p.seq_lens = seq_lens;
   p.q_start = q_start;
@@ -602,6 +597,13 @@ extern "C" int cafd_attn_prefill(const void* q, const void* k_cache, const void*
   p.lambda = lambda; p.out_scale = out_scale; p.eps = eps;
   p.sink = sink; p.gate = static_cast<const __nv_bfloat16*>(gate); p.gate_ld = gate_ld;
   p.q_head_stride = kHD;
+  cudaStream_t st = static_cast<cudaStream_t>(s);
+  const bool turn = cap > 0.f || v_table || out_scale != 1.f;
+  if (splits > 1 && (!scratch || splits > kPairSplits || !attn_prefill_paired(Hq, Hkv, maps, turn))) return -10;
+  if (attn_prefill_paired(Hq, Hkv, maps, turn)) {
+    const CUtensorMap m[5] = {tq, tk, tv, tq, tq};
+    return attn_pair(m, p, false, num_seqs, max_q_len, scratch, splits > 1 ? splits : 1, st);
+  }
   static bool attr = false;
   if (!attr) {
     CAFD_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmem));
@@ -610,9 +612,8 @@ extern "C" int cafd_attn_prefill(const void* q, const void* k_cache, const void*
     attr = true;
   }
   dim3 grid((max_q_len + kBQ - 1) / kBQ, Hq, num_seqs);
-  cudaStream_t st = static_cast<cudaStream_t>(s);
   if (maps == 2) launch_pdl(attn_prefill_kernel<false, 2>, grid, dim3(kPrefillThreads), kPrefillSmem, st, tq, tk, tv, tq, tq, p);
-  else if (cap > 0.f || v_table || out_scale != 1.f) launch_pdl(attn_prefill_kernel<false, 1, true>, grid, dim3(kPrefillThreads), kPrefillSmem, st, tq, tk, tv, tq, tq, p);
+  else if (turn) launch_pdl(attn_prefill_kernel<false, 1, true>, grid, dim3(kPrefillThreads), kPrefillSmem, st, tq, tk, tv, tq, tq, p);
   else launch_pdl(attn_prefill_kernel<false, 1>, grid, dim3(kPrefillThreads), kPrefillSmem, st, tq, tk, tv, tq, tq, p);
   return static_cast<int>(cudaGetLastError());
 }
@@ -661,6 +662,10 @@ extern "C" int cafd_attn_prefill_mla(const void* q_nope, int q_pitch, int q_head
   p.window = window;
   p.ldo = ldo;
   p.kv_tmp_start = kv_tmp_start; p.q_head_stride = q_head_stride; p.qr_head_stride = qr_head_stride; p.qr_col0 = qr_col0;
+  if (max_q_len > kBQ) {
+    const CUtensorMap m[5] = {tq, tk, tv, tqr, tkr};
+    return attn_pair(m, p, true, num_seqs, max_q_len, nullptr, 1, static_cast<cudaStream_t>(s));
+  }
   static bool attr = false;
   if (!attr) {
     CAFD_CHECK_CUDA(cudaFuncSetAttribute(attn_prefill_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrefillSmemRope));

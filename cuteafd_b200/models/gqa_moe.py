@@ -34,6 +34,7 @@ class Batch:
     prefill: bool
     last_rows: torch.Tensor | None = None   # rows whose logits are wanted (None = all)
     fresh: bool = False                     # prefill of a single sequence from position 0 (no earlier context in the cache)
+    kv_tokens: int = 0                      # the longest sequence's length after this step, where the host knows it
     # media rows: (row indices int64 [m], embeddings [m, hidden] bf16), both on the device; those rows of the input
     # take the tower's output instead of the embedding table's row (eager prefill only)
     embeds: tuple | None = None
@@ -210,6 +211,7 @@ class GqaMoeEngine:
     fused = None                 # class defaults: subclasses with their own constructor never take the fused step
     _fused_rows = 0
     _fused_checked = False
+    _prompt_shares = None
     embed_rows = None            # [max_tokens, hidden] staging of a host-resident embedding table's rows (None = table on the GPU)
 
     def __init__(self, cfg: ModelConfig, weights: GqaMoeWeights, kv: KvCache, max_tokens: int, max_seqs: int = 64,
@@ -273,6 +275,12 @@ class GqaMoeEngine:
             self.launches += 1
         return out
 
+    def _prompt_scratch(self, floats: int) -> torch.Tensor:
+        """fp32 room of a prompt's shares of keys, kept and grown (apart from the decode steps', whose address captured graphs hold)."""
+        if self._prompt_shares is None or self._prompt_shares.numel() < floats:
+            self._prompt_shares = torch.empty(floats, dtype=torch.float32, device=self.device)
+        return self._prompt_shares
+
     # ---- pieces ---------------------------------------------------------------------------------
     def _attention(self, i: int, T: int, b: Batch) -> None:
         cfg, L, ws = self.cfg, self.W.layers[i], self.ws
@@ -281,9 +289,13 @@ class GqaMoeEngine:
                      self.kv.v[i], cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.rms_eps, cfg.rope_interleaved,
                      bias=L.bqkv)
         if b.prefill:
+            S = b.page_table.shape[0]
+            # (a window's keys are few)
+            splits = 1 if cfg.window_of(i) else K.attn_prefill_splits(S, b.max_q_len, b.kv_tokens, cfg.num_heads, cfg.num_kv_heads)
             K.attn_prefill(ws.q[:T], self.kv.k[i], self.kv.v[i], b.page_table, b.seq_lens, b.q_start, ws.attn[:T],
-                           b.max_q_len, window=cfg.window_of(i))
-            self.launches += 3
+                           b.max_q_len, window=cfg.window_of(i), splits=splits,
+                           scratch=self._prompt_scratch(K.attn_prefill_scratch_floats(T, cfg.num_heads, splits)) if splits > 1 else None)
+            self.launches += 3 + (1 if splits > 1 else 0)
         else:
             S, max_pages = b.page_table.shape
             q_per_tile = 16 // (cfg.num_heads // cfg.num_kv_heads)

@@ -563,21 +563,33 @@ def attn_decode_scratch_floats(num_seqs: int, max_q_len: int, Hq: int, Hkv: int,
     return int(_n.cuda_lib().cafd_attn_decode_scratch_floats(num_seqs, tiles, Hkv, splits))
 
 
+def attn_prefill_splits(num_seqs: int, max_q_len: int, kv_tokens: int, Hq: int, Hkv: int) -> int:
+    """Shares that a prompt step's keys are cut into, at most ``kv_tokens`` for a sequence (1 in the batch-invariant form)."""
+    return int(_n.cuda_lib().cafd_attn_prefill_splits(num_seqs, max_q_len, kv_tokens, Hq, Hkv, num_sms()))
+
+
+def attn_prefill_scratch_floats(total_q: int, Hq: int, splits: int) -> int:
+    return int(_n.cuda_lib().cafd_attn_prefill_scratch_floats(total_q, Hq, splits))
+
+
 def attn_prefill(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, page_table: torch.Tensor,
                  seq_lens: torch.Tensor, q_start: torch.Tensor, out: torch.Tensor, max_q_len: int,
                  scale: float | None = None, window: int = 0, keep: int = 0, maps: int = 1, lam: float = 0.0, out_scale: float = 1.0,
                  eps: float = 0.0, sink: torch.Tensor | None = None, gate: torch.Tensor | None = None, cap: float = 0.0,
-                 v_table: torch.Tensor | None = None) -> torch.Tensor:
-    """Prompt attention; the arguments mean what they mean for ``attn_decode``."""
+                 v_table: torch.Tensor | None = None, splits: int = 1, scratch: torch.Tensor | None = None) -> torch.Tensor:
+    """Prompt attention; the arguments mean what they mean for ``attn_decode``, ``splits`` and ``scratch`` come from
+    ``attn_prefill_splits`` / ``attn_prefill_scratch_floats``."""
     T, Hq, D = q.shape
     num_pages, Hkv = k_cache.shape[0], k_cache.shape[1]
     num_seqs, max_pages = page_table.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    assert splits == 1 or (scratch is not None and scratch.dtype == torch.float32 and scratch.numel() >= attn_prefill_scratch_floats(T, Hq, splits))
     _n.check(_n.cuda_lib().cafd_attn_prefill(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), page_table.data_ptr(),
                                              seq_lens.data_ptr(), q_start.data_ptr(), out.data_ptr(),
                                              status_word(q.device).data_ptr(), T, num_seqs, max_q_len, num_pages,
                                              max_pages, Hq, Hkv, D, scale, int(window), int(keep), _attn_out(q, out, maps), maps, lam,
-                                             out_scale, eps, _ptr(sink), *_gate(gate, q, Hq), cap, _ptr(v_table), _stream()), "attn_prefill")
+                                             out_scale, eps, _ptr(sink), *_gate(gate, q, Hq), cap, _ptr(v_table), _ptr(scratch), splits,
+                                             _stream()), "attn_prefill")
     return out
 
 

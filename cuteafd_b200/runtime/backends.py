@@ -360,7 +360,7 @@ class EngineBackend:
         b.upload()
         self._stage_embeddings(b.tokens[0][:n])
         batch = Batch(b.tokens[1][:n], b.positions[1][:n], b.slots[1][:n], b.page_table[1].view(1, self.max_pages),
-                      b.seq_lens[1][:1], b.q_start[1][:2], n, True, b.last_rows[1][:1], fresh=start == 0)
+                      b.seq_lens[1][:1], b.q_start[1][:2], n, True, b.last_rows[1][:1], fresh=start == 0, kv_tokens=start + n)
         if ov is not None:
             dev = self.engine.device
             batch.embeds = (torch.tensor(ov[0], dtype=torch.long).to(dev), ov[1].to(dev, torch.bfloat16))

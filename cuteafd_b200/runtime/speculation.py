@@ -474,7 +474,8 @@ class EngineDraftModel:
             b.upload()
             every = all_rows and n <= rows_cap
             batch = Batch(b.tokens[1][:n], b.positions[1][:n], b.slots[1][:n], b.page_table[1].view(1, self.max_pages),
-                          b.seq_lens[1][:1], b.q_start[1][:2], n, True, None if every else b.last_rows[1][:1], fresh=start == 0)
+                          b.seq_lens[1][:1], b.q_start[1][:2], n, True, None if every else b.last_rows[1][:1], fresh=start == 0,
+                          kv_tokens=start + n)
             out = self.eng.forward(batch)
             seq.tokens.extend(part)
             seq.kv_len = start + n

@@ -137,3 +137,12 @@ def test_w8_rules():
     from cuteafd_b200.parallel.moe_exchange import w8_expands, w8_tile_rows
     assert [w8_tile_rows(n * 32, 8, 256) for n in (1, 20, 21, 48, 49, 300)] == [32, 32, 64, 64, 128, 128]
     assert not w8_expands(512 * 16, 16) and w8_expands(512 * 16 + 1, 16)
+
+
+def test_prompt_share_rules():
+    from cuteafd_b200._native import lib as n
+    f = n.cuda_lib().cafd_attn_prefill_splits
+    assert f(1, 512, 16896, 32, 4, 148) == 2 and f(1, 65, 16449, 32, 4, 148) == 8
+    assert f(1, 300, 1300, 32, 4, 148) == 1 and f(1, 8192, 8192, 32, 4, 148) == 1 and f(1, 777, 777, 32, 4, 148) == 1
+    assert f(1, 512, 16896, 24, 8, 148) == 1                        # an odd number of heads shares a kv head
+    assert f(1, 512, 0, 32, 4, 148) == 1                            # the host doesn't know the lengths

@@ -50,8 +50,8 @@ def test_expanded_in_the_tile(tile, H, I):
         a, b = rows @ deq[0][e].T, rows @ deq[1][e].T
         h = (torch.nn.functional.silu(a.double()) * b).to(torch.bfloat16).float()
         ref = h.double() @ deq[2][e].double().T
-        # the rounding of the result, and the fc1 outputs that fp32 sums in another order round the other way: half a unit of bf16 (2^-9) of
-        # the larger ones of I terms of random sign each
+        # the rounding of the result (2^-8 of it), and the fc1 outputs that fp32 sums in another order round the other way: a unit of bf16 (2^-7)
+        # of a few of them, taken as half of the largest term
         bound = 2.0 ** -8 * ref.abs() + 2.0 ** -8 * (h.double().abs().max() * deq[2][e].abs().max())
         assert ((out[ids == e].double() - ref).abs() <= bound).all(), e
 
