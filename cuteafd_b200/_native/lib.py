@@ -233,6 +233,8 @@ def cuda_lib():
         _sig(lib, "cafd_moe_combine", [P, P, P, P, P, I, I, I, P, I, P, P, P])
         _sig(lib, "cafd_attn_decode_scratch_floats", [I, I, I, I], C.c_longlong)
         _sig(lib, "cafd_attn_decode", [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, I, I, F, F, F, P, P, I, F, P, P])
+        _sig(lib, "cafd_attn_step_splits", [I, I, I, I, I, I])
+        _sig(lib, "cafd_attn_step", [P, P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, F, I, I, I, P])
         _sig(lib, "cafd_attn_decode_partial", [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, P])
         _sig(lib, "cafd_attn_merge", [P, P, P, I, I, I, I, I, P])
         _sig(lib, "cafd_set_fixed_kv_split", [I])

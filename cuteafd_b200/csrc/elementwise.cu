@@ -7,6 +7,7 @@
 // ties to the lowest id and NaN never selected).
 #include "cafd_api.h"
 #include "common.cuh"
+#include "rope.cuh"
 
 namespace cafd {
 
@@ -91,7 +92,6 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint4* __restrict__ 
 // ---- q/k head norm + RoPE + paged KV write (GQA) ----------------------------------------------------
 // qkv [T, (Hq + 2 Hkv) * D] from the fused projection.  One warp per (token, head).  D == 128.
 // q_out [T, Hq, D]; K/V pages [num_pages, page, Hkv, D]; slot[t] = page * page_size + offset.
-// Rounding points follow the oracle: norm -> bf16 -> rope (fp32) -> bf16.
 // kHeads: heads of one token that a warp does.  The angles are the expensive part (two sincosf at large arguments per lane) and are the
 // token's, not the head's, so a prompt chunk takes up to eight heads per warp, a token's heads shared out evenly and all loads of a warp in
 // flight at once: 8192 tokens of 32 + 2 x 4 heads 87 -> 48 us.  A step short of warps takes one.
@@ -127,27 +127,14 @@ __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __
     rb_[i] = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane);
   }
   const int slot = slots[t];
-  float s0 = 0.f, c0 = 1.f, s1 = 0.f, c1 = 1.f;
-  if (h_lo < Hq + Hkv) {
-    // pairs: whole head interleaved (2i, 2i+1), lane l holds pairs l and 32+l; whole head in halves (i, i+64), i = 2l and 2l+1;
-    // half a head interleaved, pair l; half a head in halves (i, i+32), lanes 0..15 hold i = 2l, 2l+1, lanes 16..31 their partners
-    const float pos = static_cast<float>(positions[t]);
-    const int f0 = interleaved ? lane : rot == 64 ? (2 * lane) & 31 : 2 * lane;
-    const int f1 = interleaved ? 32 + lane : f0 + 1;
-    sincosf(pos * inv_freq[f0], &s0, &c0);
-    if (!(interleaved && rot == 64)) sincosf(pos * inv_freq[f1], &s1, &c1);
-  }
+  HeadAngles ang{0.f, 1.f, 0.f, 1.f};
+  if (h_lo < Hq + Hkv) ang = head_angles(static_cast<float>(positions[t]), inv_freq, lane, interleaved, rot);
 #pragma unroll
   for (int i = 0; i < kHeads; ++i) {
     const int h = h_lo + i;
     if (h >= h_hi) return;
     uint32_t a = ra_[i], b = rb_[i];
-    if (bias) {
-      const uint32_t ba = *reinterpret_cast<const uint32_t*>(bias + h * D + 2 * lane);
-      const uint32_t bb = *reinterpret_cast<const uint32_t*>(bias + h * D + 64 + 2 * lane);
-      a = pack_bf16(bf16_lo(a) + bf16_lo(ba), bf16_hi(a) + bf16_hi(ba));
-      b = pack_bf16(bf16_lo(b) + bf16_lo(bb), bf16_hi(b) + bf16_hi(bb));
-    }
+    if (bias) head_bias(a, b, bias + h * D, lane);
     if (h >= Hq + Hkv) {  // V: plain copy into the cache
       if (slot >= 0) {
         // cache layout [page, kv head, 64 tokens, D]: one (page, head) tile is 16 KB of contiguous memory
@@ -157,36 +144,8 @@ __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __
       }
       continue;
     }
-    float x0 = bf16_lo(a), x1 = bf16_hi(a), x2 = bf16_lo(b), x3 = bf16_hi(b);
     const bool is_q = h < Hq;
-    const __nv_bfloat16* nw = is_q ? q_norm_w : k_norm_w;
-    if (nw) {
-      const float ss = warp_sum(x0 * x0 + x1 * x1 + x2 * x2 + x3 * x3);
-      const float inv = rsqrtf(ss / static_cast<float>(D) + eps);
-      const uint32_t wa = *reinterpret_cast<const uint32_t*>(nw + 2 * lane);
-      const uint32_t wb = *reinterpret_cast<const uint32_t*>(nw + 64 + 2 * lane);
-      const uint32_t ra = pack_bf16(x0 * inv * bf16_lo(wa), x1 * inv * bf16_hi(wa));
-      const uint32_t rb = pack_bf16(x2 * inv * bf16_lo(wb), x3 * inv * bf16_hi(wb));
-      x0 = bf16_lo(ra); x1 = bf16_hi(ra); x2 = bf16_lo(rb); x3 = bf16_hi(rb);
-    }
-    float y0, y1, y2, y3;
-    if (rot == 64) {
-      y2 = x2; y3 = x3;
-      if (interleaved) {
-        y0 = x0 * c0 - x1 * s0; y1 = x0 * s0 + x1 * c0;
-      } else {
-        const float p0 = __shfl_xor_sync(0xffffffffu, x0, 16), p1 = __shfl_xor_sync(0xffffffffu, x1, 16);
-        if (lane < 16) { y0 = x0 * c0 - p0 * s0; y1 = x1 * c1 - p1 * s1; }
-        else           { y0 = p0 * s0 + x0 * c0; y1 = p1 * s1 + x1 * c1; }
-      }
-    } else if (interleaved) {
-      y0 = x0 * c0 - x1 * s0; y1 = x0 * s0 + x1 * c0;
-      y2 = x2 * c1 - x3 * s1; y3 = x2 * s1 + x3 * c1;
-    } else {
-      y0 = x0 * c0 - x2 * s0; y2 = x0 * s0 + x2 * c0;
-      y1 = x1 * c1 - x3 * s1; y3 = x1 * s1 + x3 * c1;
-    }
-    const uint32_t oa = pack_bf16(y0, y1), ob = pack_bf16(y2, y3);
+    head_norm_rope(a, b, is_q ? q_norm_w : k_norm_w, eps, ang, lane, interleaved, rot);
     __nv_bfloat16* dst;
     if (is_q) {
       dst = q_out + (static_cast<size_t>(t) * Hq + h) * D;
@@ -194,8 +153,8 @@ __global__ void __launch_bounds__(128) qk_rope_kv_kernel(const __nv_bfloat16* __
       if (slot < 0) continue;
       dst = k_cache + ((static_cast<size_t>(slot >> 6) * Hkv + (h - Hq)) * 64 + (slot & 63)) * D;
     }
-    *reinterpret_cast<uint32_t*>(dst + 2 * lane) = oa;
-    *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = ob;
+    *reinterpret_cast<uint32_t*>(dst + 2 * lane) = a;
+    *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = b;
   }
 }
 

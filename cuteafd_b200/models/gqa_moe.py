@@ -285,11 +285,20 @@ class GqaMoeEngine:
     def _attention(self, i: int, T: int, b: Batch) -> None:
         cfg, L, ws = self.cfg, self.W.layers[i], self.ws
         K.linear(ws.x[:T], L.wqkv, out=ws.qkv[:T], resident=True)
+        S, max_pages = b.page_table.shape
+        step = 0 if b.prefill or b.max_q_len != 1 else K.attn_step_splits(S, max_pages, cfg.num_heads, cfg.num_kv_heads, cfg.window_of(i))
+        if step:
+            # rotation, cache write, attention and the merge of its splits in one launch
+            K.attn_step(ws.qkv[:T], L.q_norm, L.k_norm, self.inv_freq, b.positions, b.slots, self.kv.k[i], self.kv.v[i], b.page_table,
+                        b.seq_lens, b.q_start, ws.attn[:T], cfg.num_heads, cfg.rms_eps, cfg.rope_interleaved, step, bias=L.bqkv,
+                        window=cfg.window_of(i), resident=True)
+            K.linear(ws.attn[:T].view(T, -1), L.wo, out=ws.h[:T], residual=ws.h[:T], resident=True)
+            self.launches += 3
+            return
         K.qk_rope_kv(ws.qkv[:T], L.q_norm, L.k_norm, self.inv_freq, b.positions, b.slots, ws.q[:T], self.kv.k[i],
                      self.kv.v[i], cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.rms_eps, cfg.rope_interleaved,
                      bias=L.bqkv)
         if b.prefill:
-            S = b.page_table.shape[0]
             # (a window's keys are few)
             splits = 1 if cfg.window_of(i) else K.attn_prefill_splits(S, b.max_q_len, b.kv_tokens, cfg.num_heads, cfg.num_kv_heads)
             K.attn_prefill(ws.q[:T], self.kv.k[i], self.kv.v[i], b.page_table, b.seq_lens, b.q_start, ws.attn[:T],
@@ -297,7 +306,6 @@ class GqaMoeEngine:
                            scratch=self._prompt_scratch(K.attn_prefill_scratch_floats(T, cfg.num_heads, splits)) if splits > 1 else None)
             self.launches += 3 + (1 if splits > 1 else 0)
         else:
-            S, max_pages = b.page_table.shape
             q_per_tile = 16 // (cfg.num_heads // cfg.num_kv_heads)
             tiles = (b.max_q_len + q_per_tile - 1) // q_per_tile
             splits = K.kv_splits_fixed(max_pages) if self.fixed_kv_split else K.attn_decode_splits(S, tiles, cfg.num_kv_heads, max_pages, cfg.window_of(i))

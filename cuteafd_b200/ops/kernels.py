@@ -532,6 +532,29 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, p
     return out
 
 
+def attn_step_splits(num_seqs: int, max_pages: int, Hq: int, Hkv: int, window: int = 0) -> int:
+    """Blocks per (sequence, kv head) of a plain decode step's one-launch attention (``attn_step``); 0 = not that form."""
+    return int(_n.cuda_lib().cafd_attn_step_splits(num_seqs, max_pages, Hq, Hkv, int(window), num_sms()))
+
+
+def attn_step(qkv: torch.Tensor, q_norm: torch.Tensor | None, k_norm: torch.Tensor | None, inv_freq: torch.Tensor, positions: torch.Tensor,
+              slots: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, page_table: torch.Tensor, seq_lens: torch.Tensor,
+              q_start: torch.Tensor, out: torch.Tensor, Hq: int, eps: float, interleaved: bool, splits: int, *, bias: torch.Tensor | None = None,
+              scale: float | None = None, window: int = 0, resident: bool = False) -> torch.Tensor:
+    """Decode step of one new token per sequence: ``qk_rope_kv`` and ``attn_decode`` of its fused projection rows in one launch, ``splits`` from
+    ``attn_step_splits``.  ``resident``: tables, lengths and the tokens cached before this step are not written by the kernel launched last on
+    this stream."""
+    Hkv, D = k_cache.shape[1], k_cache.shape[3]
+    S, max_pages = page_table.shape
+    assert qkv.is_contiguous() and qkv.shape[1] == (Hq + 2 * Hkv) * D and out.is_contiguous() and out.shape[0] == qkv.shape[0]
+    _n.check(_n.cuda_lib().cafd_attn_step(qkv.data_ptr(), _ptr(q_norm), _ptr(k_norm), _ptr(bias), inv_freq.data_ptr(), positions.data_ptr(),
+                                          slots.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), page_table.data_ptr(), seq_lens.data_ptr(),
+                                          q_start.data_ptr(), out.data_ptr(), Hq * D, S, max_pages, Hq, Hkv, D, 2 * inv_freq.shape[0],
+                                          int(interleaved), eps, scale if scale is not None else 1.0 / math.sqrt(D), int(window), splits,
+                                          int(resident), _stream()), "attn_step")
+    return out
+
+
 def attn_decode_partial(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, page_table: torch.Tensor,
                         seq_lens: torch.Tensor, kv_base: torch.Tensor, q_start: torch.Tensor, peer_scratch: list[int], my_rank: int,
                         max_q_len: int, splits: int, scale: float | None = None) -> None:

@@ -146,3 +146,14 @@ def test_prompt_share_rules():
     assert f(1, 300, 1300, 32, 4, 148) == 1 and f(1, 8192, 8192, 32, 4, 148) == 1 and f(1, 777, 777, 32, 4, 148) == 1
     assert f(1, 512, 16896, 24, 8, 148) == 1                        # an odd number of heads shares a kv head
     assert f(1, 512, 0, 32, 4, 148) == 1                            # the host doesn't know the lengths
+
+
+def test_step_attention_rules():
+    from cuteafd_b200._native import lib as n
+    f = n.cuda_lib().cafd_attn_step_splits
+    for s, pages, hkv in ((1, 129, 4), (8, 129, 4), (32, 129, 4), (3, 8, 4), (1, 1, 1), (300, 3, 8)):
+        got = f(s, pages, 4 * hkv, hkv, 0, 148)
+        assert 1 <= got <= min(16, pages)
+    assert [f(r, 129, 32, 4, 0, 148) for r in (1, 4, 8, 16, 32)] == [16, 16, 10, 5, 6] and f(32, 8, 32, 4, 0, 148) == 2
+    assert f(1, 4000, 32, 4, 0, 148) == 0 and f(1, 4000, 32, 4, 512, 148) > 0           # a long context of one row; a window of it
+    assert f(1, 129, 136, 4, 0, 148) == 0                                               # 34 heads to a kv head
