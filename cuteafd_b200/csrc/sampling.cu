@@ -13,11 +13,14 @@
 // One cluster of one to eight blocks per row, each with its share of the vocabulary in shared memory as
 // order-preserving 32-bit keys.  What bounds the kernel is the number of dependent passes, not the
 // 0.6 MB a row is read once: with one block per row, walking the row from L2 in every pass, eight
-// rows of 151936 took 371 us and 32 rows of 129280 666 us, now 27 and 35 us.  One histogram over
+// rows of 151936 took 371 us and 32 rows of 129280 666 us, then 27 and 35 us, with the quick pass 18
+// (top-k 50) and 33 (top-p 0.9).  One histogram over
 // (maximum - value) in steps of 1/8 says how far down the first filter can reach; the tokens above
 // that line, a few hundred for the settings that chats use, are gathered into one block, sorted,
-// and all filters and the draw are prefix sums over the sorted list.  When more than 2048 tokens
-// are above the line the selections are four-level radix descents over the keys in the cluster.
+// and all filters and the draw are prefix sums over the sorted list.  The shared atomics of that
+// histogram, up to four to a token, were the longest part: where the threads' best tokens can say
+// beforehand which tokens may matter (the quick pass), the others meet none.  When more than 2048
+// tokens are above the line the selections are four-level radix descents over the keys in the cluster.
 //
 // Reference counterparts: native/shared/cuda/sampling_gpu.cu (row parameters and status codes
 // sampling_gpu.h:82-120), semantics in rust/crates/cuteafd-core/src/target_sampling.rs:9-215.
@@ -31,6 +34,13 @@ namespace cg = cooperative_groups;
 constexpr int kSampleThreads = 512;              // at 64 registers a thread two blocks share an SM: 32 rows are one wave (1024 threads: two waves, 67 us)
 constexpr int kSampleBins = 256;
 constexpr int kSampleList = 2048;                // tokens that the sorted list holds
+constexpr int kSampleNear = 1024;                // threads' best tokens above the quick pass's line
+// Tokens of a block's slice from which the quick pass gains more than its barriers cost: with top-k, and without.  Without it / with it, us: 8 rows of
+// 32000 (slices of 4000), top-k 50, 14.7 / 14.9, top-p 0.9 14.6 / 17.1; 4 of 50000 16.6 / 15.2 and 16.3 / 18.3; 20 of 100000 30 / 24 and 30.5 / 27.7; 8 of
+// 151936 27.7 / 18.2 and 28.0 / 23.9, flat rows of them 29.7 / 20.0 and 103 / 97.5.  Without top-k a row's threads must be more than a list holds to
+// show that it is flat: eight blocks (256 flat rows of 32000 on two blocks each 251 / 302).
+constexpr int kSampleQuickK = 6 * 1024, kSampleQuick = 12 * 1024;
+constexpr int kSampleNearList = 1024;            // tokens above it that a block notes
 constexpr int kSampleSmemKeys = 48 * 1024;       // keys of a slice kept in shared memory; longer slices are read again in every pass
 constexpr int kSampleKeysPair = 20 * 1024;       // up to this many two blocks share an SM
 constexpr int kLimbKeys = 1 << 17;               // slice length up to which 15-bit limbs of the masses add up in 32 bits
@@ -74,6 +84,9 @@ struct SampleHist {
 struct SampleShared {
   SampleHist hist[2];
   unsigned long long list[kSampleList];       // key << 32 | ~id: descending = the order
+  int near_id[kSampleNearList];               // places of the slice's tokens above the quick pass's line
+  unsigned long long near_mass[kSampleThreads / 32], row_mass;      // this block's share of the row's mass
+  int n_near, near_bin, near_flat;
   unsigned long long scan[32];
   int counts[32];
   float red_v[32];
@@ -81,7 +94,8 @@ struct SampleShared {
   float row_v;
   int row_i, row_c, row_bad;                  // this block's share of the row's maximum, argmax, allowed tokens, non-finite logits
   int n_list, ties, pick_id, bin;
-  unsigned long long tie_mass, acc_m;
+  unsigned long long tie_mass, acc_m, level_acc[2], level_total;      // of a descent: sum above the level's bin, and the whole
+  int level_bin[2];
   unsigned int acc_c;
 };
 
@@ -184,6 +198,7 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
     const int shift = 24 - 8 * level;
     SampleHist& h = sh.hist[level & 1];      // last read two levels ago, before the barrier of the level between
     hist_clear(h);
+    if (tid == 0) { sh.level_bin[level & 1] = 0; sh.level_acc[level & 1] = acc; }
     __syncthreads();
     for (int j = tid; j < s.n; j += kSampleThreads) {
       const uint32_t key = s.key(j);
@@ -201,21 +216,16 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
     const unsigned long long v = by_mass ? m : c;
     const unsigned long long incl = block_scan(v, sh.scan);
     if (level == 0) {
+      if (tid == kSampleThreads - 1) sh.level_total = incl;
       __syncthreads();
-      if (tid == kSampleThreads - 1) sh.acc_m = incl;
-      __syncthreads();
-      const unsigned long long total = sh.acc_m;
+      const unsigned long long total = sh.level_total;
       if (by_mass) target = mass_target(frac, strict, total);
       else target = min(max(1ull, static_cast<unsigned long long>(count_target)), max(1ull, total));
     }
+    if (tid < kSampleBins && v > 0 && acc + incl >= target && acc + incl - v < target) { sh.level_bin[level & 1] = b; sh.level_acc[level & 1] = acc + incl - v; }
     __syncthreads();
-    if (tid == 0) { sh.bin = 0; sh.acc_m = acc; }
-    __syncthreads();
-    if (tid < kSampleBins && v > 0 && acc + incl >= target && acc + incl - v < target) { sh.bin = b; sh.acc_m = acc + incl - v; }
-    __syncthreads();
-    acc = sh.acc_m;
-    prefix = (prefix << 8) | static_cast<uint32_t>(sh.bin);
-    __syncthreads();
+    acc = sh.level_acc[level & 1];
+    prefix = (prefix << 8) | static_cast<uint32_t>(sh.level_bin[level & 1]);
   }
   // ties of the pivot value: how many are needed, then the id of that tie (ascending ids: blocks in rank order, a thread a run of ids)
   const int chunk = (s.n + kSampleThreads - 1) / kSampleThreads;
@@ -250,10 +260,59 @@ __device__ Cut select_prefix(cg::cluster_group& cluster, const SampleSlice& s, C
       }
     }
   }
-  cluster.sync();
-  const Cut out{prefix, sh.pick_id};
-  cluster.sync();        // nobody's next call overwrites what another block still reads
-  return out;
+  cluster.sync();        // (what another block reads of this call is read: a next call writes it behind barriers of its own)
+  return Cut{prefix, sh.pick_id};
+}
+
+// All filters and the draw on the L tokens of sh.list (unsorted), of which the first nk in order are candidates; all_m: the row's mass.  One block.
+__device__ int pick_from_list(SampleShared& sh, int L, int nk, bool use_k, bool use_p, unsigned long long all_m, float top_p, double u, float maxp,
+                              int best_id) {
+  const int tid = threadIdx.x;
+  int pow2 = 2;
+  while (pow2 < L) pow2 <<= 1;
+  for (int j = L + tid; j < pow2; j += kSampleThreads) sh.list[j] = 0ull;
+  __syncthreads();
+  for (int k = 2; k <= pow2; k <<= 1)        // bitonic, descending
+    for (int d = k >> 1; d > 0; d >>= 1) {
+      for (int t = tid; t < pow2 / 2; t += kSampleThreads) {
+        const int i = 2 * t - (t & (d - 1)), o = i + d;
+        const unsigned long long a = sh.list[i], b = sh.list[o];
+        if ((a < b) == ((i & k) == 0)) { sh.list[i] = b; sh.list[o] = a; }
+      }
+      __syncthreads();
+    }
+  constexpr int kPer = kSampleList / kSampleThreads;
+  unsigned long long c[kPer];                // masses, then cumulative masses, at this thread's places of the list
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) {
+    const int i = kPer * tid + q;
+    c[q] = i < nk ? mass_of(key_value(static_cast<uint32_t>(sh.list[i] >> 32)), maxp) : 0ull;
+    if (q) c[q] += c[q - 1];
+  }
+  const unsigned long long own = c[kPer - 1], incl = block_scan(own, sh.scan);
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) c[q] += incl - own;
+  const unsigned long long before = incl - own;
+  if (tid == kSampleThreads - 1) sh.acc_m = use_k ? incl : all_m;
+  __syncthreads();
+  unsigned long long total = sh.acc_m;
+  if (use_p) {
+    const unsigned long long t = mass_target(static_cast<double>(top_p), false, total);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+      if (c[q] >= t && (q ? c[q - 1] : before) < t) sh.acc_m = c[q];
+    __syncthreads();
+    total = sh.acc_m;
+  }
+  const unsigned long long t = mass_target(u, true, total);
+  if (tid == 0) sh.pick_id = best_id;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < kPer; ++q)
+    if (c[q] >= t && (q ? c[q - 1] : before) < t) sh.pick_id = static_cast<int>(0xffffffffu - static_cast<uint32_t>(sh.list[kPer * tid + q]));
+  __syncthreads();
+  return sh.pick_id;
 }
 
 template <int kC>
@@ -280,6 +339,8 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   // ---- pass A: validation, max, lowest-id argmax; the logits stay in shared memory ---------------------
   float best = -INFINITY; int bi = 0x7fffffff; int cnt = 0, bad = 0;
   const bool greedy = rp.temperature < kGreedyEps || rp.top_k == 1, keep = in_smem && !greedy;
+  const bool use_k = rp.top_k > 0 && rp.top_k < V, use_p = rp.top_p < 1.0f;
+  const bool quick_pass = keep && (use_k ? slice >= kSampleQuickK : kC == 8 && slice >= kSampleQuick);
   auto take = [&](int i, float v, bool allowed) {
     const bool finite = isfinite(v);
     cnt += allowed;
@@ -347,6 +408,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
       take(id0 + j, v[q], in[q]);
     }
   }
+  const float mine = best;                      // this thread's best token
   for (int o = 16; o; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
@@ -356,7 +418,8 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   }
   if (lane == 0) { sh.red_v[wid] = best; sh.red_i[wid] = bi; sh.red_c[wid] = cnt; sh.red_bad[wid] = bad; }
   hist_clear(sh.hist[0]);
-  if (tid == 0) { sh.n_list = 0; sh.bin = kSampleBins - 1; }
+  if (quick_pass) hist_clear(sh.hist[1]);
+  if (tid == 0) { sh.n_list = 0; sh.n_near = 0; sh.bin = kSampleBins - 1; }
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < kSampleThreads / 32; ++w) {
@@ -390,51 +453,198 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
   s.maxp = best / rp.temperature;
   s.use_minp = rp.min_p > 0.f;
   s.thresh = s.use_minp ? s.maxp + static_cast<float>(log(static_cast<double>(rp.min_p))) : -INFINITY;
+  float uf = splitmix_uniform(rp.seed, rp.position);
+  uf = fminf(fmaxf(uf, 0.f), 0.99999994f);
+  const double u = static_cast<double>(uf);
+  int token = bi;
+  bool flat = false;
+  if (quick_pass) {
+    // ---- quick pass.  The best tokens of the row's threads, some 4096, give a line: above it are top-k tokens at least or, without top-k, most
+    // of those tokens' mass.  Only tokens above it meet a histogram and are noted; of the others what counts, without top-k, is their mass,
+    // which needs no atomics.  Where the first filter reaches no further than the line, the noted tokens are all there is to sort; a row too
+    // flat for that is left to the passes over all tokens.
+    const bool masses = !use_k;
+    if (mine > -INFINITY) {
+      const float xp = key_value(order_key(mine / s.temp));
+      if (!s.use_minp || xp >= s.thresh) {
+        const int b = s.bin(xp);
+        atomicAdd(&sh.hist[1].cnt[b], 1u);
+        if (masses) hist_add_mass(sh.hist[1], b, mass_of(xp, s.maxp), wide);
+      }
+    }
+    cluster.sync();
+    unsigned int bc = 0;
+    unsigned long long bm = 0;
+    if (tid < kSampleBins) hist_total<kC>(cluster, sh.hist[1], tid, wide, bc, bm);
+    const unsigned int tc = block_scan(bc, reinterpret_cast<unsigned int*>(sh.counts));
+    const unsigned long long tm = masses ? block_scan(bm, sh.scan) : 0ull;
+    if (tid == 0) { sh.near_bin = -1; sh.near_flat = 0; }
+    if (tid == kSampleThreads - 1) { sh.acc_m = tm; sh.acc_c = tc; }
+    __syncthreads();
+    if (tid < kSampleBins && bc > 0) {
+      if (masses) {
+        // the threads' tokens hold most of the mass where it is concentrated: a line at a quarter of what may be left below, of theirs
+        const double goal = use_p ? static_cast<double>(rp.top_p) : u, all = static_cast<double>(sh.acc_m), want = (0.75 + 0.25 * goal) * all;
+        if (tc <= kSampleNear && static_cast<double>(tm) >= want && static_cast<double>(tm - bm) < want) sh.near_bin = tid;
+        // more of them than a list holds reach the goal: so do more tokens, and nothing is asked about lists
+        if (tc > kSampleList && static_cast<double>(tm) >= goal * all && static_cast<double>(tm - bm) < goal * all) sh.near_flat = 1;
+      } else if (tc <= kSampleNear) {
+        const unsigned int k = static_cast<unsigned int>(rp.top_k);
+        if (tc >= k && tc - bc < k) sh.near_bin = tid;
+        else if (tc < k && tc == sh.acc_c) sh.near_bin = kSampleBins - 1;       // few threads have any candidate: all of them
+      }
+    }
+    __syncthreads();
+    flat = sh.near_flat != 0;
+    const int near = sh.near_bin;
+    const bool try_near = near >= 0;
+    if (try_near) {
+      unsigned long long mass = 0;
+      // below this no token is in the bins down to the line, or passes min_p (x / temperature, the bin and the threshold round once each)
+      const float slack = 0.1f * s.temp + 1e-6f * fabsf(best);
+      const float least = s.use_minp ? s.thresh * s.temp - 1e-6f * fabsf(s.thresh * s.temp) - slack : -INFINITY;
+      const float cut = fmaxf(least, near < kSampleBins - 1 ? best - static_cast<float>(near + 1) * 0.125f * s.temp - slack : -INFINITY);
+      auto visit = [&](int j, float xv, bool in) {
+        if (!in || xv < (masses ? least : cut)) return;
+        const float xp = s.temp == 1.0f ? xv : xv / s.temp;
+        if (s.use_minp && !(xp >= s.thresh)) return;
+        if (masses) mass += mass_of(xp, s.maxp);
+        if (xv < cut) return;
+        const float value = key_value(order_key(xp));      // one zero
+        const int b = s.bin(value);
+        if (b > near) return;
+        atomicAdd(&sh.hist[0].cnt[b], 1u);
+        if (masses) hist_add_mass(sh.hist[0], b, mass_of(value, s.maxp), wide);
+        const int at = atomicAdd(&sh.n_near, 1);
+        if (at < kSampleNearList) sh.near_id[at] = j;
+      };
+      for (int c = tid; c < (n + 3) / 4; c += kSampleThreads) {
+        const uint4 v = reinterpret_cast<const uint4*>(sm_keys)[c];
+        const int i = id0 + 4 * c;
+        uint32_t in = 0xfu;
+        if (mask) {
+          in = 0;
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (4 * c + e < n) in |= ((mask[(i + e) >> 5] >> ((i + e) & 31)) & 1u) << e;
+        }
+        visit(4 * c, __uint_as_float(v.x), in & 1u);
+        visit(4 * c + 1, __uint_as_float(v.y), (in & 2u) && 4 * c + 1 < n);
+        visit(4 * c + 2, __uint_as_float(v.z), (in & 4u) && 4 * c + 2 < n);
+        visit(4 * c + 3, __uint_as_float(v.w), (in & 8u) && 4 * c + 3 < n);
+      }
+      if (masses)
+        for (int o = 16; o; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+      if (lane == 0) sh.near_mass[wid] = mass;
+      __syncthreads();
+      if (tid == 0) {
+        for (int w = 1; w < kSampleThreads / 32; ++w) mass += sh.near_mass[w];
+        sh.row_mass = mass;
+      }
+      cluster.sync();
+      unsigned long long all_m = 0;
+      bool quick = true;
+#pragma unroll
+      for (int r = 0; r < kC; ++r) {
+        const SampleShared* o = cluster.map_shared_rank(&sh, r);
+        all_m += o->row_mass;
+        quick &= o->n_near <= kSampleNearList;
+      }
+      bc = 0; bm = 0;
+      if (tid < kSampleBins) hist_total<kC>(cluster, sh.hist[0], tid, wide, bc, bm);
+      const unsigned int cc = block_scan(bc, reinterpret_cast<unsigned int*>(sh.counts));
+      const unsigned long long cm = masses ? block_scan(bm, sh.scan) : 0ull;
+      if (tid == kSampleThreads - 1) { sh.bin = -1; sh.acc_c = cc; }
+      __syncthreads();
+      // (with top-k, fewer than k tokens down to the line are all candidates)
+      const unsigned long long first = use_k ? min(static_cast<unsigned long long>(rp.top_k), static_cast<unsigned long long>(sh.acc_c))
+                                             : mass_target(use_p ? static_cast<double>(rp.top_p) : u, !use_p, all_m);
+      __syncthreads();
+      if (tid < kSampleBins) {
+        const unsigned long long at = use_k ? cc : cm, own = use_k ? bc : bm;
+        if (own > 0 && at >= first && at - own < first) { sh.bin = tid; sh.acc_c = cc; }
+      }
+      __syncthreads();
+      const int line = sh.bin;
+      const int above = static_cast<int>(sh.acc_c);
+      if (quick && line >= 0 && above <= kSampleList) {
+        // every block hands its tokens down to the line to block 0, whose list they share out among themselves (its order does not matter:
+        // the list is sorted)
+        unsigned long long* list = cluster.map_shared_rank(sh.list, 0);
+        int* count = cluster.map_shared_rank(&sh.n_list, 0);
+        const int n_near = sh.n_near;
+        for (int e0 = 0; e0 < n_near; e0 += kSampleThreads) {
+          const int e = e0 + tid;
+          uint32_t key = 0;
+          int jn = 0;
+          if (e < n_near) {
+            jn = sh.near_id[e];
+            key = order_key(__uint_as_float(sm_keys[jn]) / s.temp);
+          }
+          const bool in = key && s.bin(key_value(key)) <= line;
+          const unsigned who = __ballot_sync(0xffffffffu, in);
+          int at = 0;
+          if (lane == 0 && who) at = atomicAdd(count, __popc(who));
+          at = __shfl_sync(0xffffffffu, at, 0) + __popc(who & ((1u << lane) - 1u));
+          if (in) list[at] = (static_cast<unsigned long long>(key) << 32) | (0xffffffffu - static_cast<uint32_t>(id0 + jn));
+        }
+        cluster.sync();
+        if (rank > 0) return;
+        token = pick_from_list(sh, above, use_k ? static_cast<int>(first) : above, use_k, use_p, all_m, rp.top_p, u, s.maxp, bi);
+        if (tid == 0) { out_token[out_row] = token; out_status[out_row] = kSampleOk; }
+        return;
+      }
+      cluster.sync();                            // every block has read what is cleared now
+      hist_clear(sh.hist[0]);
+    }
+    if (tid == 0) sh.bin = kSampleBins - 1;
+    __syncthreads();
+  }
 #pragma unroll 4
   for (int j = tid; j < n; j += kSampleThreads) {
     uint32_t key;
     if (in_smem) {
       const int i = id0 + j;
-      const float xp = __uint_as_float(sm_keys[j]) / s.temp;
+      const float x0 = __uint_as_float(sm_keys[j]), xp = s.temp == 1.0f ? x0 : x0 / s.temp;
       const bool out = (mask && !((mask[i >> 5] >> (i & 31)) & 1u)) || (s.use_minp && !(xp >= s.thresh));
       key = out ? 0u : order_key(xp);
       sm_keys[j] = key;
     } else {
       key = s.make(j);
     }
-    if (!key) continue;
+    if (!key || flat) continue;
     const float xp = key_value(key);
     const int b = s.bin(xp);
     atomicAdd(&sh.hist[0].cnt[b], 1u);
-    hist_add_mass(sh.hist[0], b, mass_of(xp, s.maxp), wide);
+    if (!use_k) hist_add_mass(sh.hist[0], b, mass_of(xp, s.maxp), wide);      // (with top-k the tokens in the cut give their own mass)
   }
   if (in_smem) s.keys = sm_keys;
-  cluster.sync();
-  const bool use_k = rp.top_k > 0 && rp.top_k < V, use_p = rp.top_p < 1.0f;
-  float uf = splitmix_uniform(rp.seed, rp.position);
-  uf = fminf(fmaxf(uf, 0.f), 0.99999994f);
-  const double u = static_cast<double>(uf);
-  unsigned int bc = 0;
-  unsigned long long bm = 0;
-  if (tid < kSampleBins) hist_total<kC>(cluster, sh.hist[0], tid, wide, bc, bm);
-  const unsigned int cc = block_scan(bc, reinterpret_cast<unsigned int*>(sh.counts));
-  const unsigned long long cm = block_scan(bm, sh.scan);
-  if (tid == kSampleThreads - 1) { sh.acc_c = cc; sh.acc_m = cm; }
-  __syncthreads();
-  const unsigned int all_c = sh.acc_c;
-  const unsigned long long all_m = sh.acc_m;
-  __syncthreads();
-  // the first filter that applies (else the draw) says how far down the order anything can be picked
-  const unsigned long long first = use_k ? min(static_cast<unsigned long long>(rp.top_k), static_cast<unsigned long long>(all_c))
-                                         : mass_target(use_p ? static_cast<double>(rp.top_p) : u, !use_p, all_m);
-  if (tid < kSampleBins) {
-    const unsigned long long at = use_k ? cc : cm, own = use_k ? bc : bm;
-    if (own > 0 && at >= first && at - own < first) { sh.bin = tid; sh.acc_c = cc; }
+  int line = kSampleBins - 1;
+  unsigned int above = kSampleList + 1;
+  unsigned long long first = 0, all_m = 0;
+  if (!flat) {
+    cluster.sync();
+    unsigned int bc = 0;
+    unsigned long long bm = 0;
+    if (tid < kSampleBins) hist_total<kC>(cluster, sh.hist[0], tid, wide, bc, bm);
+    const unsigned int cc = block_scan(bc, reinterpret_cast<unsigned int*>(sh.counts));
+    const unsigned long long cm = block_scan(bm, sh.scan);
+    if (tid == kSampleThreads - 1) { sh.acc_c = cc; sh.acc_m = cm; }
+    __syncthreads();
+    const unsigned int all_c = sh.acc_c;
+    all_m = sh.acc_m;
+    __syncthreads();
+    // the first filter that applies (else the draw) says how far down the order anything can be picked
+    first = use_k ? min(static_cast<unsigned long long>(rp.top_k), static_cast<unsigned long long>(all_c))
+                                           : mass_target(use_p ? static_cast<double>(rp.top_p) : u, !use_p, all_m);
+    if (tid < kSampleBins) {
+      const unsigned long long at = use_k ? cc : cm, own = use_k ? bc : bm;
+      if (own > 0 && at >= first && at - own < first) { sh.bin = tid; sh.acc_c = cc; }
+    }
+    __syncthreads();
+    line = sh.bin;
+    above = sh.acc_c;
   }
-  __syncthreads();
-  const int line = sh.bin;
-  const unsigned int above = sh.acc_c;
-  int token = bi;
   if (above <= kSampleList) {
     // block 0 gathers in place, the others hand their shares over through its shared memory
     for (int j = tid; j < n; j += kSampleThreads) {
@@ -453,55 +663,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(const float
     }
     cluster.sync();
     if (rank > 0) return;                      // block 0's memory is what the others wrote to; nobody reads theirs any more
-    const int L = static_cast<int>(above);
-    int pow2 = 2;
-    while (pow2 < L) pow2 <<= 1;
-    for (int j = L + tid; j < pow2; j += kSampleThreads) sh.list[j] = 0ull;
-    __syncthreads();
-    for (int k = 2; k <= pow2; k <<= 1)        // bitonic, descending
-      for (int d = k >> 1; d > 0; d >>= 1) {
-        for (int t = tid; t < pow2 / 2; t += kSampleThreads) {
-          const int i = 2 * t - (t & (d - 1)), o = i + d;
-          const unsigned long long a = sh.list[i], b = sh.list[o];
-          if ((a < b) == ((i & k) == 0)) { sh.list[i] = b; sh.list[o] = a; }
-        }
-        __syncthreads();
-      }
-    const int nk = use_k ? static_cast<int>(first) : L;
-    constexpr int kPer = kSampleList / kSampleThreads;
-    unsigned long long c[kPer];                // masses, then cumulative masses, at this thread's places of the list
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      const int i = kPer * tid + q;
-      c[q] = i < nk ? mass_of(key_value(static_cast<uint32_t>(sh.list[i] >> 32)), s.maxp) : 0ull;
-      if (q) c[q] += c[q - 1];
-    }
-    const unsigned long long own = c[kPer - 1], incl = block_scan(own, sh.scan);
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) c[q] += incl - own;
-    const unsigned long long before = incl - own;
-    if (tid == kSampleThreads - 1) sh.acc_m = use_k ? incl : all_m;
-    __syncthreads();
-    unsigned long long total = sh.acc_m;
-    if (use_p) {
-      const unsigned long long t = mass_target(static_cast<double>(rp.top_p), false, total);
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < kPer; ++q)
-        if (c[q] >= t && (q ? c[q - 1] : before) < t) sh.acc_m = c[q];
-      __syncthreads();
-      total = sh.acc_m;
-    }
-    const unsigned long long t = mass_target(u, true, total);
-    if (tid == 0) sh.pick_id = bi;
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kPer; ++q)
-      if (c[q] >= t && (q ? c[q - 1] : before) < t) sh.pick_id = static_cast<int>(0xffffffffu - static_cast<uint32_t>(sh.list[kPer * tid + q]));
-    __syncthreads();
-    token = sh.pick_id;
+    token = pick_from_list(sh, static_cast<int>(above), use_k ? static_cast<int>(first) : static_cast<int>(above), use_k, use_p, all_m, rp.top_p, u, s.maxp, bi);
   } else {
-    cluster.sync();                            // every block has read the histograms that the descents reuse
+    if (!flat) cluster.sync();                 // every block has read the histograms that the descents reuse
     Cut cut{0u, 0x7fffffff};
     if (use_k) cut = select_prefix<kC>(cluster, s, cut, false, 0.0, false, rp.top_k, wide, sh);
     if (use_p) cut = select_prefix<kC>(cluster, s, cut, true, static_cast<double>(rp.top_p), false, 0, wide, sh);
@@ -542,7 +706,7 @@ template <int kC>
 static int launch_sample(const SampleCall& c, cudaStream_t st) {
   // a slice starts at a multiple of four tokens
   const int slice = c.V <= 0 ? 0 : kC == 1 ? c.V : static_cast<int>((static_cast<long long>(c.V) + 4 * kC - 1) / (4 * kC)) * 4;
-  const size_t smem = slice <= kSampleSmemKeys ? static_cast<size_t>(slice) * 4 : 0;
+  const size_t smem = slice <= kSampleSmemKeys ? (static_cast<size_t>(slice) + 3) / 4 * 16 : 0;      // read four keys at a time
   CAFD_CHECK_CUDA(cudaFuncSetAttribute(sample_rows_kernel<kC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmemKeys * 4));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(c.n) * kC);

@@ -173,3 +173,32 @@ def test_sample_rows_of_any_alignment(n, V, ld, first):
     some = list(range(0, n, 1 if n < 10 else 23))
     want, status = select_rows(on_host[some].contiguous(), [params[i] for i in some], some, [allowed[:V] if i % 2 else None for i in some])
     assert not st.any() and status == [0] * len(some) and tok[some].tolist() == want
+
+
+@pytest.mark.parametrize("V", [4097, 60011, 151936])
+@pytest.mark.parametrize("shape", ["peaked", "flat", "steps", "one thread", "negative"])
+def test_lines_from_the_threads_best_tokens(V, shape):
+    """Rows whose candidates are few and near, too many, tied over whole bins, or all in neighbouring tokens, under every order of filters."""
+    from cuteafd_b200.ops import kernels as K
+    from cuteafd_b200.runtime.sampling import SamplingParams, select_rows
+    g = torch.Generator().manual_seed(V)
+    params = [SamplingParams(temperature=t, top_k=k, top_p=p, min_p=m, seed=7 * i)
+              for i, (t, k, p, m) in enumerate([(1.0, None, 0.9, 0.0), (0.7, 50, 0.95, 0.0), (0.6, 1000, 1.0, 0.0), (1.0, 4000, 0.9, 0.0), (1.5, None, 1.0, 0.0),
+                                                (0.8, 20, 0.8, 0.05), (1.0, None, 0.99, 0.1), (0.05, 50, 0.9, 0.0), (2.0, None, 0.3, 0.0)])]
+    n = len(params)
+    x = torch.randn(n, V, generator=g) * 2
+    if shape == "peaked":
+        x[:, torch.randperm(V, generator=g)[:300]] += 9
+    elif shape == "flat":
+        x *= 0.05
+    elif shape == "steps":
+        x = (x * 2).round() / 2                                   # values on the bins' edges, ties everywhere
+    elif shape == "one thread":
+        x[:, 1000:3000] += 8                                      # 2000 neighbours: more than a block notes
+    else:
+        x = x.abs().neg() * 50 - 1000
+    want, status = select_rows(x, params, list(range(n)), [None] * n)
+    rows = K.pack_sample_rows(params, list(range(n))).cuda()
+    tok, st = torch.full((n,), -7, dtype=torch.int32, device="cuda"), torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    K.sample_rows(x.cuda(), rows, tok, st)
+    assert st.tolist() == status and tok.tolist() == want
