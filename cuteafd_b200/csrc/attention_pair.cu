@@ -207,7 +207,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int tpos0 = pos0 + (kRope ? i * kBQ : 0), rowpos = tpos0 + row;
     const uint32_t tS = tmem + i * 128 + (static_cast<uint32_t>(quad * 32) << 16), tO = tS + 256;
     const int ni = i ? n1 : n0;
-    float m_run = -INFINITY, l_run = 0.f;
+    float m_run = -INFINITY, l_half[2] = {0.f, 0.f};        // sums of the tiles' two column halves, as the one-tile kernel keeps them
     const uint64_t scale2 = pair_f32x2(p.scale_log2, p.scale_log2);
     bool ok = true;
     for (int j = 0; j < ni; ++j) {
@@ -233,7 +233,8 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
         for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(mx4[k], __uint_as_float(r[c + k]));
       }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;       // scale > 0
+      // (rounded up to bf16, the one-tile kernel's reference: the same bits)
+      const float mx = __bfloat162float(__float2bfloat16_ru(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])))) * p.scale_log2;       // scale > 0
       // the reference maximum only moves by more than 8 (factor 256): P stays within the range of bf16 and fp32 and O is rescaled rarely;
       // O and the running sum share the reference, so the quotient is exact all the same
       const float m_new = (mx > m_run + 8.0f) ? mx : m_run;
@@ -262,15 +263,17 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
               : "=f"(e0), "=f"(e1) : "r"(r[c + k]), "r"(r[c + k + 1]), "l"(scale2), "l"(nbase2));
           e0 = fast_exp2(e0);
           e1 = fast_exp2(e1);
-          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[(k >> 1) & 1]) : "l"(pair_f32x2(e0, e1)));
+          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c >> 6]) : "l"(pair_f32x2(e0, e1)));
           pk[k >> 1] = pack_bf16(e0, e1);
         }
         tmem_st_32x16(tS + (c >> 1), pk);
       }
-      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[0]) : "l"(sum[1]));
-      float s0, s1;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sum[0]));
-      l_run = l_run * corr + (s0 + s1);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float s0, s1;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sum[h]));
+        l_half[h] = l_half[h] * corr + (s0 + s1);
+      }
       m_run = m_new;
       tmem_st_wait();
       tc_fence_before();
@@ -278,6 +281,7 @@ attn_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (lane == 0) mbar_arrive(&p_ready[i]);
     }
     // ---- epilogue: O / l, or this share's O, maximum and sum ------------------------------------------
+    float l_run = l_half[0] + l_half[1];
     if (ni > 0) ok = ok && mbar_wait_warp(&o_full[i], 0, p.status, kTimeoutTmemFull);
     tc_fence_after();
     const bool row_ok = rows0 + row < q_len;

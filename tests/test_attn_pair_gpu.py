@@ -100,3 +100,14 @@ def test_rows_of_one_head(T):
         w, vh = torch.softmax(s, -1), v[:T, h * 128:(h + 1) * 128].double()
         ref[:, h], mass[:, h] = w @ vh, w @ vh.abs()
     _close(out, ref, mass)
+
+
+@pytest.mark.parametrize("T,ctx,window", [(777, 0, 0), (130, 400, 0), (513, 200, 300)])
+def test_bits_of_the_one_tile_kernel(T, ctx, window):
+    """A kv head of two heads (two tiles per block) and the same head given twice (one tile per block)."""
+    from cuteafd_b200.ops import kernels as K
+    q, kc, vc, table, sl, qs, _, _ = _case([T], [ctx], 2, 1, seed=T)
+    one, two = torch.empty_like(q), torch.empty_like(q)
+    K.attn_prefill(q, kc, vc, table, sl, qs, two, T, window=window)
+    K.attn_prefill(q, kc.repeat(1, 2, 1, 1), vc.repeat(1, 2, 1, 1), table, sl, qs, one, T, window=window)
+    assert torch.equal(one, two)
