@@ -224,20 +224,31 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   if (wide_hist) {
     // Wide form (prefill-sized steps): moe_count_kernel left one histogram per 256-entry chunk; turn them into each
     // chunk's first position per expert.  moe_scatter_kernel places the entries afterwards.
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-      int run = 0;
-      for (int g0 = 0; g0 < wide_chunks; g0 += 8) {
-        int c[8];
+    // `parts` threads share an expert's chunks (one thread per expert walked 256 chunks of 65536 entries in 15 us)
+    const int parts = min(static_cast<int>(blockDim.x) / e_stride, kPlanSlots / e_stride), per = (wide_chunks + parts - 1) / parts;
+    const int e = static_cast<int>(threadIdx.x) % e_stride, part = static_cast<int>(threadIdx.x) / e_stride;
+    const bool mine = part < parts && e < E;
+    const int g_lo = min(wide_chunks, part * per), g_hi = min(wide_chunks, g_lo + per);
+    auto walk = [&](int run, bool put) {
+      for (int g0 = g_lo; g0 < g_hi; g0 += 16) {
+        int c[16];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) c[k] = g0 + k < wide_chunks ? wide_hist[static_cast<size_t>(g0 + k) * e_stride + e] : 0;
+        for (int k = 0; k < 16; ++k) c[k] = g0 + k < g_hi ? wide_hist[static_cast<size_t>(g0 + k) * e_stride + e] : 0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (g0 + k < wide_chunks) wide_hist[static_cast<size_t>(g0 + k) * e_stride + e] = run;
+        for (int k = 0; k < 16; ++k) {
+          if (put && g0 + k < g_hi) wide_hist[static_cast<size_t>(g0 + k) * e_stride + e] = run;
           run += c[k];
         }
       }
-      counts[e] = run;
-      cursor[e] = 0;
+      return run;
+    };
+    if (mine) wcount(part, e) = walk(0, false);
+    __syncthreads();
+    if (mine) {
+      int before = 0, all = 0;
+      for (int q = 0; q < parts; ++q) { const int v = wcount(q, e); if (q < part) before += v; all += v; }
+      walk(before, true);
+      if (part == 0) { counts[e] = all; cursor[e] = 0; }
     }
     __syncthreads();
   } else {
@@ -371,14 +382,15 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    const int r = rank_of[e];
-    int* row_dst = L.meta[r] + kMetaHeader + 2 * L.max_tiles;
-    const int padded = (counts[e] + tile_rows - 1) / tile_rows * tile_rows;
-    for (int pos = counts[e]; pos < padded; ++pos)
-      if (seg_off[e] + pos < L.max_rows) row_dst[seg_off[e] + pos] = -1;
-    if (expert_count_out) expert_count_out[e] += counts[e];
+  // rows of padding behind every segment: a warp per expert, or a thread where they are few (tiles of 128: 6 us less than a thread each)
+  const int step = tile_rows >= 64 ? 32 : 1, first = tile_rows >= 64 ? lane_id : 0;
+  for (int e = tile_rows >= 64 ? warp_id : threadIdx.x; e < E; e += tile_rows >= 64 ? static_cast<int>(blockDim.x >> 5) : blockDim.x) {
+    int* row_dst = L.meta[rank_of[e]] + kMetaHeader + 2 * L.max_tiles + seg_off[e];
+    const int padded = min((counts[e] + tile_rows - 1) / tile_rows * tile_rows, L.max_rows - seg_off[e]);
+    for (int pos = counts[e] + first; pos < padded; pos += step) row_dst[pos] = -1;
   }
+  if (expert_count_out)
+    for (int e = threadIdx.x; e < E; e += blockDim.x) expert_count_out[e] += counts[e];
   if (x) {
     __syncthreads();                      // dest_row of every entry is written (same block: visible after the barrier)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -416,6 +428,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
         }
       }
     }
+    if (!L.flag[0]) return;               // the rows' reader is this stream's next kernel
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -509,9 +522,8 @@ __global__ void __launch_bounds__(256) moe_dispatch_kernel(const uint4* __restri
                                                            uint32_t* done_counter, int wpt) {
   pdl_wait();
   pdl_trigger();
-  // wpt = 1 (large steps): one warp per token, the row is read once (eight 16-byte loads in flight per lane) and
-  // stored to each of its top_k destinations.  wpt = 8 (decode-sized steps): a block per token whose eight warps
-  // share the row's columns: a handful of tokens then spreads over as many SMs as there are tokens instead of one.
+  // The row is read once, its warps share the columns (up to eight 16-byte loads in flight per lane), and stored to each of its top_k
+  // destinations.
   const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int t = gw / wpt, sub = gw - t * wpt;
   const int lane = threadIdx.x & 31;
@@ -568,6 +580,9 @@ __global__ void __launch_bounds__(256) moe_dispatch_kernel(const uint4* __restri
       }
     }
   }
+  // Without flags the rows' reader is this stream's next kernel.  (The fence of the whole system and the count of blocks took longer than the
+  // rows of a decode step.)
+  if (!L.flag[0]) return;
   __threadfence_system();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -833,7 +848,9 @@ int cafd_moe_dispatch(const void* x, const int* idx, const int* dest_row, int T,
   if (H % 8 || top_k > 32) return -10;
   if (layout->fp8 && !wire_ok(layout, H)) return -11;
   const int n = T * top_k;
-  const int wpt = T <= 64 ? 8 : 1;                       // few tokens: a block per token, its warps share the slots
+  // Warps per token: one for each is too few rows in flight.  With 1 / 2 / 4 / 8, eight destinations, us: rows of 4 KB, 256 tokens 5.7 / 3.7 / 3.1 / 4.9, 777
+  // 6.1 / 6.4 / 5.7 / 8.5, 2048 16.6 / 14.2 / 12.3 / 18.7, 8192 52.7 / 49.0 / 50.8 / 77; of 14 KB, 300 16.9 / 9.4 / 9.1 / 8.0, 3000 74 / 67 / 64 / 62.
+  const int wpt = T <= 64 || H >= 4096 ? 8 : T <= 4096 ? 4 : 2;
   const int blocks = T > 0 ? (T * wpt + 7) / 8 : 1;      // eight warps per block
   launch_pdl(moe_dispatch_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(s), static_cast<const uint4*>(x), idx, dest_row, n,
                                                                        top_k, H / 8, to_dev(layout), epoch,

@@ -305,7 +305,8 @@ class AttentionSide:
         self._rank_ptrs: list[tuple[int, int, int]] = []
 
     def bind_rank(self, r: int, slab_ptr: int, meta_ptr: int, flags_ptr: int) -> None:
-        """Record rank r's slab / meta / per-layer dispatch flag base (local or peer addresses)."""
+        """Record rank r's slab / meta / per-layer dispatch flag base (local or peer addresses; flags 0: the rows are read by later
+        kernels of the same stream only, and nothing is published)."""
         while len(self._rank_ptrs) <= r:
             self._rank_ptrs.append((0, 0, 0))
         self._rank_ptrs[r] = (slab_ptr, meta_ptr, flags_ptr)
@@ -332,7 +333,7 @@ class AttentionSide:
         if logits is not None:
             K.route_topk(logits, g.top_k, out_idx=idx, out_w=w, **route_kw)
         for r in range(g.n_expert_ranks):
-            self.layout.flag[r] = self._rank_ptrs[r][2] + 4 * layer
+            self.layout.flag[r] = self._rank_ptrs[r][2] + 4 * layer if self._rank_ptrs[r][2] else 0
         if x.dtype == torch.float32:              # rows travel as bytes: a 32-bit row is a bf16 row of twice the length
             x = x.view(torch.bfloat16)
         if (T * g.top_k <= self.FUSED_DISPATCH_ROWS and T * g.top_k * x.shape[1] * 2 <= self.FUSED_DISPATCH_BYTES
@@ -359,7 +360,7 @@ class LocalExchange:
         self.geo = geo
         self.att = AttentionSide(geo, device, dtype=dtype)
         self.exp = ExpertSide(geo, device, dtype=dtype)
-        self.att.bind_rank(0, self.exp.slab.data_ptr(), self.exp.meta.data_ptr(), self.exp.flags.data_ptr())
+        self.att.bind_rank(0, self.exp.slab.data_ptr(), self.exp.meta.data_ptr(), 0)
         self.epoch = torch.zeros(1, dtype=torch.int32, device=device)
 
     def skinny(self, x: torch.Tensor, w_gate: torch.Tensor, w_down: torch.Tensor) -> bool:
