@@ -22,8 +22,8 @@ __device__ __forceinline__ float route_value(uint32_t k) {
 }
 
 // ---- router -------------------------------------------------------------------------------------
-// One warp routes one token: `row` points at its E router logits in global memory.
-template <int kPerLane>
+// One warp routes one token: `row` points at its E router logits in global memory, or (kShared) in the block's own shared memory.
+template <int kPerLane, bool kShared = false>
 __device__ __forceinline__ void route_row(const float* row, const float* __restrict__ bias, int* __restrict__ out_idx,
                                           float* __restrict__ out_w, int t, int E, int top_k, int scoring, int num_groups,
                                           int topk_groups, int normalize, float routed_scale, int group_max = 0) {
@@ -33,7 +33,7 @@ __device__ __forceinline__ void route_row(const float* row, const float* __restr
 #pragma unroll
   for (int j = 0; j < kPerLane; ++j) {
     const int e = j * 32 + lane;
-    score[j] = e < E ? __ldcg(row + e) : -INFINITY;     // written by other blocks (or an earlier kernel): skip L1
+    score[j] = e >= E ? -INFINITY : kShared ? row[e] : __ldcg(row + e);     // global: written by other blocks (or an earlier kernel), skip L1
     if (scoring == 2 && bias && e < E) score[j] += bias[e];
     mx = fmaxf(mx, score[j]);
   }

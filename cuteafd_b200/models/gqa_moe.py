@@ -372,7 +372,7 @@ class GqaMoeEngine:
         logits = None
         if fused:
             K.norm_route(ws.h[:T], L.ln2, cfg.rms_eps, L.router, ws.x[:T], self.moe.att.idx[:T], self.moe.att.w[:T], cfg.top_k,
-                         bias=L.router_bias, **self.route_kw)
+                         bias=L.router_bias, resident=True, **self.route_kw)
             self.launches += 1
         else:
             K.rmsnorm(ws.h[:T], L.ln2, cfg.rms_eps, out=ws.x[:T])

@@ -325,10 +325,11 @@ _route_scratch: dict = {}
 def norm_route(h: torch.Tensor, ln_w: torch.Tensor | None, eps: float, router_w: torch.Tensor, x_out: torch.Tensor | None, out_idx: torch.Tensor,
                out_w: torch.Tensor, top_k: int, *, scoring: str = "softmax", bias: torch.Tensor | None = None, num_groups: int = 1,
                topk_groups: int = 1, normalize: bool = True, routed_scale: float = 1.0,
-               logits_out: torch.Tensor | None = None, group_score: str = "top2") -> None:
+               logits_out: torch.Tensor | None = None, group_score: str = "top2", resident: bool = False) -> None:
     """x_out = RMSNorm(h) * ln_w, router scores x_out @ router_w.T and the top-k routing of every row in one launch
     (grid token x 8 expert groups; meant for decode-sized batches).  ``logits_out`` [T, E] fp32 receives the scores
-    (a per-device scratch is used when it is not given).  ``ln_w`` None: the rows are normalised already."""
+    (a per-device scratch is used when it is not given).  ``ln_w`` None: the rows are normalised already.  ``resident``: the kernel
+    launched last on this stream does not write the weights of the norm and the router."""
     T, H = h.shape
     E = router_w.shape[0]
     key = h.device.index
@@ -342,7 +343,7 @@ def norm_route(h: torch.Tensor, ln_w: torch.Tensor | None, eps: float, router_w:
     _n.check(_n.cuda_lib().cafd_norm_route(h.data_ptr(), _ptr(ln_w), eps, router_w.data_ptr(), _ptr(bias), _ptr(x_out),
                                            out_idx.data_ptr(), out_w.data_ptr(), buf.data_ptr(), sc[1].data_ptr(), T, H, E, top_k,
                                            SCORING[scoring], num_groups, topk_groups, int(normalize), routed_scale,
-                                           int(group_score == "max"), _stream()), "norm_route")
+                                           int(group_score == "max"), int(resident), _stream()), "norm_route")
 
 
 # Tokens up to which a step's bf16 experts run on the few-row kernel, measured with plan, dispatch and combine against the tcgen05 kernel.

@@ -428,6 +428,31 @@ def test_norm_route_matches_separate_kernels(K, E, k, scoring, groups, keep, H):
     assert torch.allclose(w[rows], w_ref[rows], rtol=2e-3, atol=1e-5)
 
 
+@pytest.mark.parametrize("E,H", [(7, 64), (8, 4096), (33, 2048), (65, 512), (127, 2056), (128, 4096), (129, 2048), (64, 4104)])
+@pytest.mark.parametrize("T", [1, 9, 10, 32, 33])
+def test_norm_route_sizes(K, E, H, T):
+    """Sizes on both sides of the lines between a cluster per token (16 blocks, 8 blocks) and blocks that meet by tickets: scores within the
+    error of an fp32 sum of the kernel's own rows, routes those of the routing kernel from these scores, weights read early or not alike."""
+    h, lw, rw = bf(T, H, seed=1), bf(H, seed=2) * 0.1 + 1.0, bf(E, H, scale=0.05, seed=3)
+    k, outs = min(E, 6), []
+    for resident, normed in ((False, False), (True, False), (True, True)):
+        x = K.rmsnorm(h, lw, 1e-6)
+        x_out = torch.zeros_like(h)
+        idx = torch.full((T, k), -1, dtype=torch.int32, device=dev()); w = torch.zeros(T, k, device=dev())
+        logits = torch.full((T, E), float("nan"), device=dev())
+        K.norm_route(x if normed else h, None if normed else lw, 1e-6, rw, None if normed else x_out, idx, w, k, logits_out=logits,
+                     resident=resident)
+        check_status(K)
+        assert normed or torch.equal(x_out, x)
+        # each lane adds H / 32 products one after another, five more additions join the lanes: (H / 32 + 5) * 2^-24 of the products' sizes
+        ref, size = x.double() @ rw.double().T, x.double().abs() @ rw.double().abs().T
+        assert ((logits - ref).abs() <= (H / 32 + 6) * 2.0 ** -24 * size).all()
+        idx2, w2 = K.route_topk(logits, k)
+        assert torch.equal(idx, idx2) and torch.equal(w, w2)
+        outs.append((logits, idx, w))
+    assert all(torch.equal(a, b) for o in outs[1:] for a, b in zip(outs[0], o))
+
+
 def test_combine_with_fused_norm(K):
     T, k, H = 7, 4, 2048
     buf, res, nw = bf(T * k, H, seed=1), bf(T, H, seed=2), bf(H, seed=3) * 0.1 + 1.0
