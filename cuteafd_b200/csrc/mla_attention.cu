@@ -7,13 +7,19 @@
 // One kernel serves decode rows, speculative-verify rows and prefill chunks; a split over the
 // KV range plus a fixed-order merge covers the decode case with few rows.
 //
-//   grid (row block, half of the 512 output dims, kv split)       192 threads
-//   warp 0   TMA: the 128 x 576 query block once (9 swizzle atoms), then 32-token KV tiles
-//            (9 atoms each, two stages) straight from the page pool
-//   warp 1   MMA: S = Q C^T (36 steps of 128x32x16), O += P V with V = the CTA's 256 latent
-//            columns read MN-major from the same tile (2 steps of 128x256x16)
-//   warps 2-5 softmax: thread = row; P goes to shared memory in the unswizzled canonical layout
-// TMEM: S double-buffered (2 x 32 columns) + O (256 columns).
+//   grid (row block, half of the 512 output dims, kv split)       320 threads
+//   warp 0   TMA: three swizzle atoms of the 128 x 576 query block, then KV tiles of a page (64 tokens, 9 atoms each, two
+//            stages) straight from the page pool; the five atoms that only the scores read are free again before the four of V
+//   warp 1   MMA: S = Q C^T (36 steps of 128x64x16, 24 of them with Q from TMEM), O += P V with V = the CTA's 256 latent
+//            columns read MN-major from the same tile (4 steps of 128x256x16)
+//   warps 2-9 six atoms of the query block into TMEM, then softmax: two threads per row, half of a tile's columns each; P goes
+//            to shared memory in the unswizzled canonical layout
+// TMEM: S (64 columns) + six query atoms (192 columns) + O (256 columns).
+//
+// Bound by a tile's chain (load, scores, softmax, PV) with two tiles in shared memory, so the query block is kept where it costs little:
+// all of it in shared memory left room for two tiles of 32 tokens, and every score product read 4 KB of queries for 1 KB of keys.  A tile
+// of 64 takes 1.6 us (32 tokens took 1.9).  128 heads, with the merge: 1 row over 8192 tokens 32.9 -> 21.9 us, 8 rows 86.9 -> 42.5, 32 rows
+// 315 -> 122, 512 prompt tokens behind 7680 3846 -> 1524, one row over 128 tokens 14.8 -> 9.6, 32 rows over 2048 listed records 154 -> 121.
 //
 // Reference counterparts: SIMT absorbed/sparse MLA kernels and the LSE state merge
 // (native/shared/cuda/attention.cu:249-925), compose of the absorbed query
@@ -27,12 +33,16 @@ namespace cafd {
 constexpr int kLat = 512, kRope = 64, kRec = kLat + kRope;     // 576 cached dims per token
 constexpr int kAtoms = kRec / 64;                             // 9 swizzle atoms along the record
 constexpr int kMlaRows = 128;
-constexpr int kKvTile = 32;
-constexpr int kQBytes = kAtoms * kMlaRows * 128;              // 147456
-constexpr int kKvBytes = kAtoms * kKvTile * 128;              // 36864
-constexpr int kPBytes = kMlaRows * kKvTile * 2;               // 8192
-constexpr int kMlaSmem = kQBytes + 2 * kKvBytes + kPBytes + 1024;
-constexpr int kMlaThreads = 192;
+constexpr int kQTmem = 6;                                     // query atoms [0, kQTmem) are in TMEM, the rest in shared memory
+constexpr int kKvTile = 64;                                   // tokens per tile: a page
+constexpr int kQBytes = (kAtoms - kQTmem) * kMlaRows * 128;   // 49152
+constexpr int kKvBytes = kAtoms * kKvTile * 128;              // 73728
+constexpr int kVBytes = 4 * kKvTile * 128;                    // the atoms that are V for this CTA
+constexpr int kPBytes = kMlaRows * kKvTile * 2;               // 16384
+constexpr int kXBytes = kMlaRows * 128;                       // one staged query atom, then the softmax's exchange
+constexpr int kMlaSmem = kQBytes + 2 * kKvBytes + kPBytes + kXBytes + 1024;
+static_assert(kQTmem == 6 && 4 * kMlaRows * 128 <= kKvBytes && kMlaRows * 128 <= kPBytes, "the query atoms on their way to TMEM");
+constexpr int kMlaThreads = 320;
 constexpr int kHalf = 256;                                    // output columns per CTA
 constexpr int kMlaPartial = kMlaRows * kHalf + 2 * kMlaRows;  // floats per (block, half, split)
 
@@ -88,8 +98,13 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* sQ = smem;
   uint8_t* sC = smem + kQBytes;                 // two stages
   uint8_t* sP = smem + kQBytes + 2 * kKvBytes;
+  uint8_t* sX = sP + kPBytes;
+  // the query atoms that go to TMEM arrive in the second stage, the probabilities' buffer and sX, all idle until then
+  auto staged = [&](int a) { return a < 4 ? sC + kKvBytes + a * (kMlaRows * 128) : a == 4 ? sP : sX; };
+  auto s_max = reinterpret_cast<float (*)[2][kMlaRows]>(sX);       // [tile parity][half of the columns][row]; sums at the end
 
-  __shared__ uint64_t q_full, c_full[2], c_empty[2], s_full[2], s_empty[2], p_ready, pv_done;
+  // of a stage: k = the five atoms that only the scores read, v = the four that PV reads as well
+  __shared__ uint64_t q_full, qt_in, qt_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_ready, pv_done;
   __shared__ uint32_t tmem_slot;
 
   pdl_wait();
@@ -118,11 +133,14 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
+    mbar_init(&qt_in, 1);
+    mbar_init(&qt_full, 256);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&c_full[i], sparse ? 32 : 1); mbar_init(&c_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128);
+      mbar_init(&k_full[i], sparse ? 32 : 1); mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], sparse ? 32 : 1); mbar_init(&v_empty[i], 1);
     }
-    mbar_init(&p_ready, 128);
+    mbar_init(&s_full, 1); mbar_init(&s_empty, 256);
+    mbar_init(&p_ready, 256);
     mbar_init(&pv_done, 1);
     mbar_fence_init();
   }
@@ -134,81 +152,124 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const uint32_t tS = tmem;          // + 32 * buffer
-  const uint32_t tO = tmem + 64;
+  const uint32_t tS = tmem;
+  const uint32_t tQ = tmem + kKvTile;          // + 32 * atom
+  const uint32_t tO = tQ + kQTmem * 32;
+
+  auto load_q = [&](int qrow) {
+    mbar_expect_tx(&qt_in, kQTmem * kMlaRows * 128);
+    for (int a = 0; a < kQTmem; ++a) tma_load_2d(staged(a), &tm_q, &qt_in, a * 64, qrow);
+    mbar_expect_tx(&q_full, kQBytes);
+    for (int a = kQTmem; a < kAtoms; ++a) tma_load_2d(sQ + (a - kQTmem) * kMlaRows * 128, &tm_q, &q_full, a * 64, qrow);
+  };
 
   if (warp == 0 && sparse) {
-    // gather producer: the whole warp copies 32 records (1152 bytes each) per tile into the swizzled
+    // gather producer: the whole warp copies 64 records (1152 bytes each) per tile into the swizzled
     // tile layout with 16-byte async copies; the copies of tile j are in flight while tile j-1 is consumed
     if (n_tiles > 0) {
       if (lane == 0) {
         tma_prefetch_desc(&tm_q);
-        mbar_expect_tx(&q_full, kQBytes);
         const int qrow = (q0 + tok0) * p.heads;
-        for (int a = 0; a < kAtoms; ++a) tma_load_2d(sQ + a * kMlaRows * 128, &tm_q, &q_full, a * 64, qrow);
+        load_q(qrow);
       }
       const int* idx = p.sparse_idx + static_cast<size_t>(q0 + tok0) * p.sparse_k;
       const int* pt = p.page_table + static_cast<size_t>(seq) * p.max_pages;
       bool ok = true;
+      auto publish = [&](int j) {
+        fence_async_smem();
+        mbar_arrive(&k_full[j & 1]);
+        mbar_arrive(&v_full[j & 1]);
+      };
+      auto copy = [](uint32_t dst, const uint8_t* src, bool have) {              // size 0: the 16 bytes are zero-filled
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have ? 16u : 0u) : "memory");
+      };
       for (int j = 0; j < n_tiles; ++j) {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        if (j > 0) {                       // publish tile j-1 before blocking: freeing a stage needs it consumed
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-          fence_async_smem();
-          mbar_arrive(&c_full[(j - 1) & 1]);
+        // tile j - 1 is published before the wait for a stage that is not free yet: freeing it needs that tile consumed
+        const bool free_now = __all_sync(0xffffffffu, mbar_try_wait(&k_empty[st], ph ^ 1) && mbar_try_wait(&v_empty[st], ph ^ 1) &&
+                                                          (j != 1 || mbar_try_wait(&qt_full, 0)));
+        if (!free_now) {
+          if (j > 0) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            publish(j - 1);
+          }
+          if (!mbar_wait(&k_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier) || !mbar_wait(&v_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier) ||
+              (j == 1 && !mbar_wait(&qt_full, 0, p.status, kTimeoutSoftmax))) {
+            ok = false;
+            break;
+          }
         }
-        if (!mbar_wait(&c_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier)) { ok = false; break; }
-        const int e = (t_begin + j) * kKvTile + lane;
-        const int pos = e < max_limit ? idx[e] : -1;
-        long long rec = -1;
-        if (pos >= 0 && (pos >> 6) < seq_pages)
-          rec = (p.gathered ? static_cast<long long>(blockIdx.x) * p.sparse_k + e
-                            : static_cast<long long>(pt[pos >> 6]) * 64 + (pos & 63)) * (kRec * 2);
+        long long rec[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int e = (t_begin + j) * kKvTile + i * 32 + lane;
+          const int pos = e < max_limit ? idx[e] : -1;
+          rec[i] = -1;
+          if (pos >= 0 && (pos >> 6) < seq_pages)
+            rec[i] = (p.gathered ? static_cast<long long>(blockIdx.x) * p.sparse_k + e
+                                 : static_cast<long long>(pt[pos >> 6]) * 64 + (pos & 63)) * (kRec * 2);
+        }
         const uint32_t dst0 = smem_u32(sC + st * kKvBytes);
-#pragma unroll 4
-        for (int c = lane; c < kKvTile * 72; c += 32) {
-          const int tok = c / 72, piece = c - tok * 72;
-          const long long r = __shfl_sync(0xffffffffu, rec, tok);
-          const uint32_t dst = dst0 + (piece >> 3) * (kKvTile * 128) + tok * 128 + (((piece & 7) ^ (tok & 7)) << 4);
-          const uint8_t* src = p.cache + (r >= 0 ? r : 0) + piece * 16;
-          const uint32_t sz = r >= 0 ? 16u : 0u;                      // size 0: the 16 bytes are zero-filled
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz) : "memory");
+        // a record's first 64 pieces of 16 bytes by two copies of the warp, the last 8 of four records by one
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+#pragma unroll 2
+          for (int t4 = 0; t4 < 32; t4 += 4) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const int tok = i * 32 + t4 + t;
+              const long long r = __shfl_sync(0xffffffffu, rec[i], t4 + t);
+              const uint8_t* src = p.cache + (r >= 0 ? r : 0) + lane * 16;
+              const uint32_t dst = dst0 + (lane >> 3) * (kKvTile * 128) + tok * 128 + (((lane & 7) ^ (tok & 7)) << 4);
+              copy(dst, src, r >= 0);
+              copy(dst + 4 * (kKvTile * 128), src + 512, r >= 0);
+            }
+            const int tok = i * 32 + t4 + (lane >> 3);
+            const long long r = __shfl_sync(0xffffffffu, rec[i], t4 + (lane >> 3));
+            copy(dst0 + 8 * (kKvTile * 128) + tok * 128 + (((lane & 7) ^ (tok & 7)) << 4), p.cache + (r >= 0 ? r : 0) + 1024 + (lane & 7) * 16, r >= 0);
+          }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        if (free_now && j > 0) {
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          publish(j - 1);
+        }
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
-      fence_async_smem();
-      if (ok) mbar_arrive(&c_full[(n_tiles - 1) & 1]);
+      if (ok) publish(n_tiles - 1);
     }
   } else if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
       tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_c);
-      mbar_expect_tx(&q_full, kQBytes);
       const int qrow = (q0 + tok0) * p.heads;
-      for (int a = 0; a < kAtoms; ++a) tma_load_2d(sQ + a * kMlaRows * 128, &tm_q, &q_full, a * 64, qrow);
+      load_q(qrow);
       mla_trace(tr, 0, 1);
       const int* pt = p.page_table + static_cast<size_t>(seq) * p.max_pages;
-      // Only two tiles fit in shared memory beside the query block, which is one tile (36 KB) in flight: far
-      // too little to cover HBM latency.  The tiles further ahead are therefore pulled into L2 early, so the
-      // load that fills a freed stage pays L2 latency only.
-      constexpr int kL2Ahead = 6;
+      // Two tiles in shared memory do not cover HBM latency: the tiles further ahead are pulled into L2 early, so the load
+      // that fills a freed stage pays L2 latency only.
+      constexpr int kL2Ahead = 3;
+      const int v0 = dh * 4;                                 // V: atoms [v0, v0 + 4)
       int pf = 2;
       for (int j = 0; j < n_tiles; ++j) {
         const int tile = t_begin + j;
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int pg_i = tile >> 1;
-        const int page = pg_i < seq_pages ? pt[pg_i] : 0;
+        const int page = tile < seq_pages ? pt[tile] : 0;
         for (; pf < n_tiles && pf <= j + kL2Ahead; ++pf) {
           const int ptile = t_begin + pf;
-          const int ppage = (ptile >> 1) < seq_pages ? pt[ptile >> 1] : 0;
-          for (int a = 0; a < kAtoms; ++a) tma_prefetch_l2_3d(&tm_c, a * 64, (ptile & 1) * kKvTile, ppage);
+          const int ppage = ptile < seq_pages ? pt[ptile] : 0;
+          for (int a = 0; a < kAtoms; ++a) tma_prefetch_l2_3d(&tm_c, a * 64, 0, ppage);
         }
-        if (!mbar_wait(&c_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier)) break;
         uint8_t* cd = sC + st * kKvBytes;
-        mbar_expect_tx(&c_full[st], kKvBytes);
-        for (int a = 0; a < kAtoms; ++a) tma_load_3d(cd + a * kKvTile * 128, &tm_c, &c_full[st], a * 64, (tile & 1) * kKvTile, page);
+        if (j == 1 && !mbar_wait(&qt_full, 0, p.status, kTimeoutSoftmax)) break;       // the queries have left the second stage
+        if (!mbar_wait(&k_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier)) break;
+        mbar_expect_tx(&k_full[st], kKvBytes - kVBytes);
+        for (int a = 0; a < kAtoms; ++a)
+          if (a < v0 || a >= v0 + 4) tma_load_3d(cd + a * kKvTile * 128, &tm_c, &k_full[st], a * 64, 0, page);
+        if (!mbar_wait(&v_empty[st], ph ^ 1, p.status, kTimeoutEmptyBarrier)) break;
+        mbar_expect_tx(&v_full[st], kVBytes);
+        for (int a = v0; a < v0 + 4; ++a) tma_load_3d(cd + a * kKvTile * 128, &tm_c, &v_full[st], a * 64, 0, page);
         mla_trace(tr, 0, 100 + j);
       }
     }
@@ -216,62 +277,86 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (n_tiles > 0) {
       constexpr uint32_t idesc_qk = make_idesc(128, kKvTile, 1, 1, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc(128, kHalf, 1, 1, 0, 1);      // B = V is MN-major
-      const uint64_t dQ = smem_desc_k_sw128(smem_u32(sQ)), dC = smem_desc_k_sw128(smem_u32(sC)), dP = smem_desc_k_noswz(smem_u32(sP), 128, 512);
+      const uint64_t dQ = smem_desc_k_sw128(smem_u32(sQ)), dC = smem_desc_k_sw128(smem_u32(sC)), dP = smem_desc_k_noswz(smem_u32(sP), 128, 1024);
       const uint64_t dV = smem_desc_mn_sw128(smem_u32(sC) + dh * 4 * (kKvTile * 128), kKvTile * 128);
-      bool ok = mbar_wait_warp(&q_full, 0, p.status, kTimeoutFullBarrier);
+      bool ok = mbar_wait_warp(&q_full, 0, p.status, kTimeoutFullBarrier) && mbar_wait_warp(&qt_full, 0, p.status, kTimeoutSoftmax);
       if (lane == 0) mla_trace(tr, 1, ok ? 1 : 2);
-      auto issue_qk = [&](int j) -> bool {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait_warp(&c_full[st], ph, p.status, kTimeoutFullBarrier)) return false;
-        if (!mbar_wait_warp(&s_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty)) return false;
+      // Scores of tile j in two parts: the atoms that only they read (loaded as soon as the previous tile but one was scored), then V's
+      // atoms (loaded as soon as that tile's PV is through).
+      auto qk = [&](int j, bool v) {
         tc_fence_after();
         if (elect_one()) {
-          const uint64_t c0 = dC + static_cast<uint64_t>(st * (kKvBytes >> 4));
+          const uint64_t c0 = dC + static_cast<uint64_t>((j & 1) * (kKvBytes >> 4));
+          // (rolled: five call sites of 36 products in line cost a short context 3 us of instruction fetches)
+          const int other = 4 - dh * 4;                      // first atom of the half that is not V
+          const int n = v ? 4 : 5;
+          uint32_t acc = v ? 1u : 0u;
+#pragma unroll 1
+          for (int i = 0; i < n; ++i) {
+            const int a = v ? dh * 4 + i : i < 4 ? other + i : 8;
+            const uint64_t b = c0 + static_cast<uint64_t>(a * (kKvTile * 128 >> 4));
+            if (a < kQTmem) {
 #pragma unroll
-          for (int a = 0; a < kAtoms; ++a)
+              for (int k4 = 0; k4 < 4; ++k4, acc = 1u) umma_f16_ts(tS, tQ + a * 32 + k4 * 8, b + (k4 * 32 >> 4), idesc_qk, acc);
+            } else {
+              const uint64_t q = dQ + static_cast<uint64_t>((a - kQTmem) * (kMlaRows * 128 >> 4));
 #pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4)
-              umma_f16(tS + st * 32, dQ + ((a * kMlaRows * 128 + k4 * 32) >> 4), c0 + ((a * kKvTile * 128 + k4 * 32) >> 4), idesc_qk,
-                       (a | k4) ? 1u : 0u);
-          umma_commit(&s_full[st]);
-          mla_trace(tr, 1, 100 + j);
+              for (int k4 = 0; k4 < 4; ++k4, acc = 1u) umma_f16(tS, q + (k4 * 32 >> 4), b + (k4 * 32 >> 4), idesc_qk, acc);
+            }
+          }
+          umma_commit(v ? &s_full : &k_empty[j & 1]);
+          if (v) mla_trace(tr, 1, 100 + j);
         }
         __syncwarp();
-        return true;
       };
-      if (ok) ok = issue_qk(0);
-      for (int j = 0; ok && j < n_tiles; ++j) {
-        // Next tile's scores go first when its data has landed (they overlap this tile's softmax); otherwise this
-        // tile's PV goes first, which frees its stage and starts the load after next that much earlier.
-        const int nst = (j + 1) & 1;
-        const uint32_t nph = ((j + 1) >> 1) & 1;
-        bool next_done = j + 1 >= n_tiles;
-        if (!next_done && __all_sync(0xffffffffu, mbar_try_wait(&c_full[nst], nph) && mbar_try_wait(&s_empty[nst], nph ^ 1))) {
-          if (!issue_qk(j + 1)) { ok = false; break; }
-          next_done = true;
-        }
-        const int st = j & 1;
-        if (!mbar_wait_warp(&p_ready, j & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+      auto pv = [&](int j) {
         tc_fence_after();
         if (elect_one()) {
+          const int st = j & 1;
           const uint64_t v0 = dV + static_cast<uint64_t>(st * (kKvBytes >> 4));
+          // a last tile of half a page: the other half's records are not read (its probabilities are zero, its bytes may be anything)
+          const bool both = (t_begin + j) * kKvTile + 32 < max_limit;
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            // A = P rows, K cores ks*2 and ks*2+1 (128 bytes apart), 8-row groups 512 bytes apart
-            // B = V: 16 kv rows per step (2 KiB), 64-column blocks 4 KiB apart, 8-row groups 1 KiB apart
-            umma_f16(tO, dP + (ks * 256 >> 4), v0 + (ks * 2048 >> 4), idesc_pv, (j | ks) ? 1u : 0u);
+          for (int ks = 0; ks < kKvTile / 16; ++ks) {
+            // A = P rows, K cores ks*2 and ks*2+1 (128 bytes apart), 8-row groups 1 KiB apart
+            // B = V: 16 kv rows per step (2 KiB), 64-column blocks 8 KiB apart, 8-row groups 1 KiB apart
+            if (ks < 2 || both) umma_f16(tO, dP + (ks * 256 >> 4), v0 + (ks * 2048 >> 4), idesc_pv, (j | ks) ? 1u : 0u);
           }
-          umma_commit(&c_empty[st]);
+          umma_commit(&v_empty[st]);
           umma_commit(&pv_done);
           mla_trace(tr, 1, 10000 + j);
         }
         __syncwarp();
-        if (!next_done && !issue_qk(j + 1)) { ok = false; break; }
+      };
+      auto ready = [&](uint64_t* bar, uint32_t phase) { return __all_sync(0xffffffffu, mbar_try_wait(bar, phase)); };
+      // Tile j + 1's scores (in two parts) and tile j's PV do not need each other: whichever has its inputs goes, the scores first, since
+      // a softmax waits for them and the PV only holds the load after next.
+      for (int j = -1; ok && j < n_tiles; ++j) {
+        const int nst = (j + 1) & 1;
+        const uint32_t nph = ((j + 1) >> 1) & 1;
+        int scored = j + 1 < n_tiles ? 0 : 2;                // parts of the next tile's scores that are issued
+        bool summed = j < 0;
+        for (int spin = 0; ok && (scored < 2 || !summed); ++spin) {
+          if (scored < 2 && (scored == 0 ? ready(&s_empty, ((j + 1) & 1) ^ 1) && ready(&k_full[nst], nph) : ready(&v_full[nst], nph))) {
+            qk(j + 1, scored == 1);
+            ++scored;
+            spin = 0;
+          } else if (!summed && ready(&p_ready, j & 1)) {
+            pv(j);
+            summed = true;
+            spin = 0;
+          } else if (spin >= 32) {                           // a bounded wait for one that needs none of the others
+            ok = !summed ? mbar_wait_warp(&p_ready, j & 1, p.status, kTimeoutSoftmax)
+                 : scored == 0 ? mbar_wait_warp(&s_empty, ((j + 1) & 1) ^ 1, p.status, kTimeoutTmemEmpty) &&
+                                     mbar_wait_warp(&k_full[nst], nph, p.status, kTimeoutFullBarrier)
+                               : mbar_wait_warp(&v_full[nst], nph, p.status, kTimeoutFullBarrier);
+          }
+        }
       }
     }
   } else {
-    const int quad = warp & 3;
+    const int quad = warp & 3, hf = (warp - 2) >> 2;       // TMEM lanes of this warp, half of the columns
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); };
     const int row = quad * 32 + lane;
     const int ti = row / p.heads;
     const bool row_valid = (tok0 + ti) < q_len && ti < tok_per_blk;
@@ -279,26 +364,53 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int low = p.window > 0 ? base_vis + tok0 + ti + 1 - p.window : 0;      // first position inside this row's window
     const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
     float m_run = -INFINITY, l_run = 0.f;
-    bool ok = true;
-    for (int j = 0; ok && j < n_tiles; ++j) {
-      const int st = j & 1;
-      const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[st], ph, p.status, kTimeoutTmemFull)) { ok = false; break; }
+    bool ok = n_tiles == 0 || mbar_wait(&qt_in, 0, p.status, kTimeoutFullBarrier);
+    if (n_tiles > 0) {                                   // three of the row's first six atoms: columns of two values
+#pragma unroll 1
+      for (int a = hf * (kQTmem / 2); a < (hf + 1) * (kQTmem / 2); ++a) {
+        uint32_t v[32];
+        const uint8_t* src = staged(a) + row * 128;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 u = *reinterpret_cast<const uint4*>(src + ((i ^ (row & 7)) << 4));
+          v[i * 4] = u.x; v[i * 4 + 1] = u.y; v[i * 4 + 2] = u.z; v[i * 4 + 3] = u.w;
+        }
+        tmem_st_32x32(tQ + a * 32 + lane_off, v);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&qt_full);
+    }
+    for (int j = 0; j < n_tiles; ++j) {
+      // (a warp whose wait ran out still meets its partner at every tile)
+      if (ok) ok = mbar_wait(&s_full, j & 1, p.status, kTimeoutTmemFull);
+      if (!ok) { pair_sync(); continue; }
       tc_fence_after();
       if (threadIdx.x == 64) mla_trace(tr, 2, 100 + j);
       uint32_t r[32];
-      tmem_ld_32x32(tS + st * 32 + lane_off, r);
+      tmem_ld_32x32(tS + hf * 32 + lane_off, r);
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(&s_empty[st]);
-      const int col0 = (t_begin + j) * kKvTile;
-      float mx = -INFINITY;
+      mbar_arrive(&s_empty);
+      const int col0 = (t_begin + j) * kKvTile + hf * 32;
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       float s[32];
+      if (__all_sync(0xffffffffu, col0 + 32 <= limit && col0 >= low)) {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        s[i] = (col0 + i < limit && col0 + i >= low) ? __uint_as_float(r[i]) * p.scale_log2 : -INFINITY;
-        mx = fmaxf(mx, s[i]);
+        for (int i = 0; i < 32; ++i) {
+          s[i] = __uint_as_float(r[i]) * p.scale_log2;
+          mx4[i & 3] = fmaxf(mx4[i & 3], s[i]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          s[i] = (col0 + i < limit && col0 + i >= low) ? __uint_as_float(r[i]) * p.scale_log2 : -INFINITY;
+          mx4[i & 3] = fmaxf(mx4[i & 3], s[i]);
+        }
       }
+      s_max[j & 1][hf][row] = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      pair_sync();
+      const float mx = fmaxf(s_max[j & 1][0][row], s_max[j & 1][1][row]);
       // The running reference m_run only moves when the tile maximum exceeds it by more than 8 (in log2
       // units), so O is rescaled rarely; P then stays below 2^8 and the final O / l is unchanged in exact
       // arithmetic because l accumulates with the same reference.
@@ -306,21 +418,22 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const float m_new = move ? mx : m_run;
       const float base = (m_new == -INFINITY) ? 0.f : m_new;
       const float corr = !move ? 1.0f : (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - base);
-      float rs = 0.f;
+      float rs2[2] = {0.f, 0.f};
       uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         const uint32_t w = pack_bf16(fast_exp2(s[i] - base), fast_exp2(s[i + 1] - base));
-        rs += bf16_lo(w) + bf16_hi(w);
+        rs2[(i >> 1) & 1] += bf16_lo(w) + bf16_hi(w);
         pk[i >> 1] = w;
       }
+      const float rs = rs2[0] + rs2[1];
       if (j > 0) {
         // P of the previous tile is still being read by its PV product until this barrier completes
-        if (!mbar_wait(&pv_done, (j - 1) & 1, p.status, kTimeoutTmemFull)) { ok = false; break; }
+        if (!mbar_wait(&pv_done, (j - 1) & 1, p.status, kTimeoutTmemFull)) { ok = false; continue; }
         tc_fence_after();
         if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll 1
-          for (int c = 0; c < kHalf; c += 32) {
+          for (int c = hf * (kHalf / 2); c < (hf + 1) * (kHalf / 2); c += 32) {
             uint32_t o[32];
             tmem_ld_32x32(tO + lane_off + c, o);
             tmem_ld_wait();
@@ -330,8 +443,8 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
       }
-      // canonical unswizzled K-major layout: core (row / 8, k / 8) at (row/8)*512 + (k/8)*128, rows 16 B apart
-      uint8_t* prow = sP + (row >> 3) * 512 + (row & 7) * 16;
+      // canonical unswizzled K-major layout: core (row / 8, k / 8) at (row/8)*1024 + (k/8)*128, rows 16 B apart
+      uint8_t* prow = sP + (row >> 3) * 1024 + (row & 7) * 16 + hf * 512;
 #pragma unroll
       for (int kc = 0; kc < 4; ++kc)
         *reinterpret_cast<uint4*>(prow + kc * 128) = make_uint4(pk[4 * kc], pk[4 * kc + 1], pk[4 * kc + 2], pk[4 * kc + 3]);
@@ -347,28 +460,40 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool have = n_tiles > 0 && ok;
     if (have) have = mbar_wait(&pv_done, (n_tiles - 1) & 1, p.status, kTimeoutTmemFull);
     tc_fence_after();
+    pair_sync();                                         // the last tile's maxima are read
+    s_max[0][hf][row] = l_run;
+    pair_sync();
+    l_run = s_max[0][0][row] + s_max[0][1][row];
     const size_t grow = p.out_tpad > 0 ? static_cast<size_t>(row % p.heads) * p.out_tpad + (q0 + tok0 + ti)
                                        : static_cast<size_t>(q0 + tok0) * p.heads + row;
     if (p.splits == 1 && p.n_peers == 0) {
       // tcgen05.ld is warp-collective: every lane loads, only valid rows store
       const float inv = (have && l_run > 0.f) ? 1.0f / l_run : 0.f;
-      __nv_bfloat16* orow = p.out + grow * kLat + dh * kHalf;
       const bool any_have = __all_sync(0xffffffffu, have);
+      // through shared memory, whose tiles are read: a row's 256 bytes leave by sixteen lanes (16 bytes of 32 rows at once took 3 us)
+      constexpr int kPitch = (kHalf / 2) * 2 + 16;                 // bytes
+      uint8_t* stage = sC + (hf * 4 + quad) * (32 * kPitch);
 #pragma unroll 1
-      for (int c = 0; c < kHalf; c += 32) {
+      for (int c = 0; c < kHalf / 2; c += 32) {
         uint32_t o[32];
-        if (any_have) { tmem_ld_32x32(tO + lane_off + c, o); tmem_ld_wait(); }
-        if (row_valid) {
+        if (any_have) { tmem_ld_32x32(tO + lane_off + hf * (kHalf / 2) + c, o); tmem_ld_wait(); }
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 q;
-            q.x = pack_bf16(any_have ? __uint_as_float(o[i]) * inv : 0.f, any_have ? __uint_as_float(o[i + 1]) * inv : 0.f);
-            q.y = pack_bf16(any_have ? __uint_as_float(o[i + 2]) * inv : 0.f, any_have ? __uint_as_float(o[i + 3]) * inv : 0.f);
-            q.z = pack_bf16(any_have ? __uint_as_float(o[i + 4]) * inv : 0.f, any_have ? __uint_as_float(o[i + 5]) * inv : 0.f);
-            q.w = pack_bf16(any_have ? __uint_as_float(o[i + 6]) * inv : 0.f, any_have ? __uint_as_float(o[i + 7]) * inv : 0.f);
-            *reinterpret_cast<uint4*>(orow + c + i) = q;
-          }
+        for (int i = 0; i < 32; i += 8) {
+          uint4 q;
+          q.x = pack_bf16(any_have ? __uint_as_float(o[i]) * inv : 0.f, any_have ? __uint_as_float(o[i + 1]) * inv : 0.f);
+          q.y = pack_bf16(any_have ? __uint_as_float(o[i + 2]) * inv : 0.f, any_have ? __uint_as_float(o[i + 3]) * inv : 0.f);
+          q.z = pack_bf16(any_have ? __uint_as_float(o[i + 4]) * inv : 0.f, any_have ? __uint_as_float(o[i + 5]) * inv : 0.f);
+          q.w = pack_bf16(any_have ? __uint_as_float(o[i + 6]) * inv : 0.f, any_have ? __uint_as_float(o[i + 7]) * inv : 0.f);
+          *reinterpret_cast<uint4*>(stage + lane * kPitch + (c + i) * 2) = q;
         }
+      }
+      const unsigned valid = __ballot_sync(0xffffffffu, row_valid);
+      __syncwarp();
+#pragma unroll 4
+      for (int r = lane >> 4; r < 32; r += 2) {
+        const long long g = __shfl_sync(0xffffffffu, static_cast<long long>(grow), r);
+        const uint4 q = *reinterpret_cast<const uint4*>(stage + r * kPitch + (lane & 15) * 16);
+        if ((valid >> r) & 1u) *reinterpret_cast<uint4*>(p.out + g * kLat + dh * kHalf + hf * (kHalf / 2) + (lane & 15) * 8) = q;
       }
     } else {
       const bool have_all = __all_sync(0xffffffffu, have);
@@ -377,7 +502,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           ? ((static_cast<size_t>(blk) * 2 + dh) * p.total_splits + p.split_offset + split) * kMlaPartial
           : ((static_cast<size_t>(blk) * 2 + dh) * p.splits + split) * kMlaPartial;
 #pragma unroll 1
-      for (int c = 0; c < kHalf; c += 32) {
+      for (int c = hf * (kHalf / 2); c < (hf + 1) * (kHalf / 2); c += 32) {
         uint32_t o[32];
         if (have_all) { tmem_ld_32x32(tO + lane_off + c, o); tmem_ld_wait(); }
         for (int d = 0; d < n_dst; ++d) {               // plain (peer) stores; the flag that publishes them follows in stream order
@@ -386,7 +511,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int i = 0; i < 32; ++i) part[static_cast<size_t>(c + i) * kMlaRows + row] = have_all ? __uint_as_float(o[i]) : 0.f;
         }
       }
-      for (int d = 0; d < n_dst; ++d) {
+      for (int d = 0; d < n_dst && hf == 0; ++d) {
         float* part = (p.n_peers > 0 ? p.peer_partial[d] : p.partial) + part_off;
         part[kMlaRows * kHalf + row] = have_all ? m_run : -INFINITY;
         part[kMlaRows * kHalf + kMlaRows + row] = have_all ? l_run : 0.f;
@@ -482,6 +607,65 @@ __global__ void __launch_bounds__(kMlaRows * kMergeGroups) mla_merge_kernel(cons
   }
 }
 
+// A few splits: the four groups take eight columns each and all splits, four at a time, so a block covers 32 columns and nothing is left to
+// add between groups.  Bound by the blocks and what each does one after another, not by bytes: at 32 row blocks of two splits the launch above
+// has 2048 blocks.  Attention and merge over 1000 tokens, 4 splits of 8 rows 23.3 -> 16.5 us, 2 of 32 rows 48.2 -> 27.4; over 8192 tokens, 9
+// splits of 8 rows 46.5 -> 42.5.  From a dozen splits on the groups' shorter chains are faster (18 of 4 rows: 28.8 us there, 32.4 here).
+constexpr int kFewSplits = 4, kFewChunks = 10;
+template <bool kOneChunk>
+__global__ void __launch_bounds__(kMlaRows * kMergeGroups) mla_merge_few_kernel(const float* __restrict__ partial, const int* __restrict__ block_seq,
+                                                                 const int* __restrict__ block_tok0, const int* __restrict__ q_start,
+                                                                 __nv_bfloat16* __restrict__ out, int heads, int splits, int out_tpad, int one_token) {
+  pdl_wait();
+  pdl_trigger();
+  const int blk = blockIdx.x, dh = blockIdx.y;
+  const int row = threadIdx.x & (kMlaRows - 1), c0 = (blockIdx.z * kMergeGroups + threadIdx.x / kMlaRows) * kMergeCols;
+  const int seq = block_seq[blk], tok0 = block_tok0[blk];
+  const int q0 = q_start[seq], q_len = q_start[seq + 1] - q0;
+  if (tok0 + row / heads >= q_len || (one_token && row >= heads)) return;
+  const float* base = partial + (static_cast<size_t>(blk) * 2 + dh) * splits * kMlaPartial + row;
+  float M = -INFINITY;
+  if (!kOneChunk)
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) M = fmaxf(M, __ldg(base + static_cast<size_t>(s) * kMlaPartial + kMlaRows * kHalf));
+  float L = 0.f, acc[kMergeCols] = {};
+#pragma unroll 1
+  for (int s0 = 0; s0 < (kOneChunk ? 1 : splits); s0 += kFewSplits) {
+    float v[kFewSplits][kMergeCols], m[kFewSplits], l[kFewSplits];
+#pragma unroll
+    for (int s = 0; s < kFewSplits; ++s) {
+      const bool have = s0 + s < splits;
+      const float* ps = base + static_cast<size_t>(s0 + s) * kMlaPartial;
+      m[s] = have ? __ldg(ps + kMlaRows * kHalf) : -INFINITY;
+      l[s] = have ? __ldg(ps + kMlaRows * kHalf + kMlaRows) : 0.f;
+#pragma unroll
+      for (int c = 0; c < kMergeCols; ++c) v[s][c] = have ? __ldg(ps + (c0 + c) * kMlaRows) : 0.f;
+    }
+    if (kOneChunk) M = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+#pragma unroll
+    for (int s = 0; s < kFewSplits; ++s) {
+      const float fac = m[s] == -INFINITY ? 0.f : exp2f(m[s] - M);
+      L += l[s] * fac;
+#pragma unroll
+      for (int c = 0; c < kMergeCols; ++c) acc[c] += v[s][c] * fac;
+    }
+  }
+  const float invL = L > 0.f ? 1.0f / L : 0.f;
+  uint32_t o[kMergeCols / 2];
+#pragma unroll
+  for (int c = 0; c < kMergeCols; c += 2) o[c / 2] = pack_bf16(acc[c] * invL, acc[c + 1] * invL);
+  const size_t grow = out_tpad > 0 ? static_cast<size_t>(row % heads) * out_tpad + (q0 + tok0 + row / heads)
+                                   : static_cast<size_t>(q0 + tok0) * heads + row;
+  *reinterpret_cast<uint4*>(out + grow * kLat + dh * kHalf + c0) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+static void launch_merge(const float* scratch, const int* block_seq, const int* block_tok0, const int* q_start, void* out, int n_blocks, int heads, int splits,
+                         int out_tpad, int one_token, cudaStream_t st) {
+  auto kern = splits <= kFewSplits ? mla_merge_few_kernel<true> : splits <= kFewChunks ? mla_merge_few_kernel<false> : mla_merge_kernel;
+  launch_pdl(kern, dim3(n_blocks, 2, kHalf / kMergeCols / (splits <= kFewChunks ? kMergeGroups : 1)), dim3(kMlaRows * kMergeGroups), 0,
+             st, scratch, block_seq, block_tok0, q_start, static_cast<__nv_bfloat16*>(out), heads, splits, out_tpad, one_token);
+}
+
 }  // namespace cafd
 
 using namespace cafd;
@@ -555,8 +739,7 @@ static int mla_attention_impl(const void* q, const void* cache, const int* page_
   cudaStream_t st = static_cast<cudaStream_t>(s);
   launch_pdl(mla_attn_kernel, dim3(n_blocks, 2, splits), dim3(kMlaThreads), kMlaSmem, st, tq, tc, p);
   if (splits > 1 && !n_peers)
-    launch_pdl(mla_merge_kernel, dim3(n_blocks, 2, kHalf / kMergeCols), dim3(kMlaRows * kMergeGroups), 0, st, static_cast<const float*>(scratch), block_seq,
-               block_tok0, q_start, static_cast<__nv_bfloat16*>(out), heads, splits, out_tpad, sparse_idx ? 1 : 0);
+    launch_merge(scratch, block_seq, block_tok0, q_start, out, n_blocks, heads, splits, out_tpad, sparse_idx ? 1 : 0, st);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -605,8 +788,7 @@ extern "C" int cafd_mla_merge(const float* scratch, const int* block_seq, const 
                               int n_blocks, int heads, int total_splits, int out_tpad, cafd_stream_t s) {
   if (n_blocks <= 0) return 0;
   if (!scratch || total_splits < 1 || total_splits > kMaxSplits || heads <= 0 || kMlaRows % heads) return -10;
-  launch_pdl(mla_merge_kernel, dim3(n_blocks, 2, kHalf / kMergeCols), dim3(kMlaRows * kMergeGroups), 0, static_cast<cudaStream_t>(s), scratch,
-             block_seq, block_tok0, q_start, static_cast<__nv_bfloat16*>(out), heads, total_splits, out_tpad, 0);
+  launch_merge(scratch, block_seq, block_tok0, q_start, out, n_blocks, heads, total_splits, out_tpad, 0, static_cast<cudaStream_t>(s));
   return static_cast<int>(cudaGetLastError());
 }
 

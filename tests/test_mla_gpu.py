@@ -83,6 +83,44 @@ def test_mla_attention(K, heads, lens, qlens, splits):
         o += n
 
 
+@pytest.mark.parametrize("heads,splits,listed,window", [(128, 1, 0, 0), (128, 2, 0, 0), (16, 4, 0, 0), (16, 5, 0, 0), (64, 10, 0, 0), (32, 11, 0, 0),
+                                                        (16, 1, 0, 70), (16, 3, 0, 33), (128, 1, 33, 0), (16, 2, 100, 0), (32, 3, 320, 0)])
+def test_mla_attention_tiles(K, heads, splits, listed, window):
+    """Contexts around the edges of a page and of half a page, one and several splits per merge form, listed records in and out of whole
+    tiles, windows that begin inside a page.  What lies in the unused half of a last page is not read."""
+    lens = [1, 31, 32, 33, 63, 64, 65, 96, 97, 128, 129, 200, 321]
+    cache, table, dense = _latent_cache(lens, seed=heads + splits)
+    for i, n in enumerate(lens):
+        if 0 < n % 64 <= 32:
+            cache[table[i, n // 64].long(), 32:] = float("nan")
+    S, dev = len(lens), _dev()
+    g = torch.Generator().manual_seed(5)
+    q = (torch.randn(S, heads, 576, generator=g) * 0.5).to(torch.bfloat16)
+    scale = 1.0 / math.sqrt(192)
+    bs, bt = K.mla_blocks([1] * S, 128 if listed else heads)
+    i32 = dict(dtype=torch.int32, device=dev)
+    pos = [torch.randperm(n, generator=g)[:listed].sort().values if listed else torch.arange(max(0, n - window) if window else 0, n) for n in lens]
+    sparse = None
+    if listed:
+        sparse = torch.full((S, listed), -1, **i32)
+        for i, x in enumerate(pos):
+            sparse[i, :len(x)] = x.to(dev, torch.int32)
+    out = torch.full((S, heads, 512), 7.0, dtype=torch.bfloat16, device=dev)
+    scratch = torch.empty(K.mla_scratch_floats(len(bs), splits), dtype=torch.float32, device=dev) if splits > 1 else None
+    K.mla_attention(q.to(dev), cache, table, torch.tensor(lens, **i32), torch.arange(S + 1, **i32), torch.tensor(bs, **i32), torch.tensor(bt, **i32),
+                    out, scale, splits, scratch, sparse_idx=sparse, window=window)
+    torch.cuda.synchronize()
+    assert K.read_status() == 0
+    for i, x in enumerate(pos):
+        c = dense[i][x].double()
+        w = torch.softmax(torch.einsum("hd,ld->hl", q[i].double(), c) * scale, -1)
+        ref, size = w @ c[:, :512], w @ c[:, :512].abs()
+        # bf16 probabilities over a sum of the same bf16 probabilities: twice half an ulp; scores of fp32 sums of 576 products of about 7 in
+        # all and the fast exponential: 2^-10; the result's own rounding
+        bound = (2 * 2.0 ** -8 + 2.0 ** -10) * size + 2.0 ** -8 * ref.abs()
+        assert ((out[i].cpu().double() - ref).abs() <= bound).all(), i
+
+
 def _mla_cfg():
     from cuteafd_b200.config import ModelConfig
     return ModelConfig(name="mla-moe-small", family="deepseek_v3", vocab_size=2048, num_layers=3, hidden=512,
