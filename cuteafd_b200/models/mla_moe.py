@@ -280,7 +280,7 @@ class MlaMoeEngine(GqaMoeEngine):
             # decode-sized step: nope / rope split, RoPE and the absorb projection in one launch
             K.mla_absorb_small(ws.q[:T], L.w_uk, self.inv_freq, b.positions, ws.q_abs[:T], heads, cfg.rope_interleaved)
         else:
-            K.mla_q_split(ws.q[:T], self.inv_freq, b.positions, q_slab, ws.q_abs[:T], heads, cfg.rope_interleaved)
+            K.mla_q_split(ws.q[:T], self.inv_freq, b.positions, None if expanded else q_slab, ws.q_abs[:T], heads, cfg.rope_interleaved)
         if expanded:
             rows = ((T + 63) // 64) * 64
             K.linear(ws.lat[:T], L.w_kb, out=ws.k_exp[:T])

@@ -779,13 +779,14 @@ def attn_prefill_mla(q_nope: torch.Tensor, q_rope: torch.Tensor, k_exp: torch.Te
     return out
 
 
-def mla_q_split(q: torch.Tensor, inv_freq: torch.Tensor, positions: torch.Tensor, slab: torch.Tensor, q_abs: torch.Tensor,
+def mla_q_split(q: torch.Tensor, inv_freq: torch.Tensor, positions: torch.Tensor, slab: torch.Tensor | None, q_abs: torch.Tensor,
                 heads: int, interleaved: bool) -> None:
-    """q [T, heads*192] -> slab [heads, t_pad, 128] (nope dims, head-major) and q_abs[:, :, 512:] (rotated rope dims)."""
+    """q [T, heads*192] -> slab [heads, t_pad, 128] (nope dims, head-major; None: they stay in q) and q_abs[:, :, 512:] (rotated rope
+    dims)."""
     T = q.shape[0]
-    assert q.shape[1] == heads * 192 and slab.shape[0] == heads and slab.shape[2] == 128
+    assert q.shape[1] == heads * 192 and (slab is None or (slab.shape[0] == heads and slab.shape[2] == 128))
     _n.check(_n.cuda_lib().cafd_mla_q_split(q.data_ptr(), q.stride(0), inv_freq.data_ptr(), positions.data_ptr(),
-                                            slab.data_ptr(), q_abs.data_ptr(), T, heads, slab.shape[1], int(interleaved),
+                                            _ptr(slab), q_abs.data_ptr(), T, heads, slab.shape[1] if slab is not None else 0, int(interleaved),
                                             _stream()), "mla_q_split")
 
 

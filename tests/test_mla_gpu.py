@@ -121,6 +121,34 @@ def test_mla_attention_tiles(K, heads, splits, listed, window):
         assert ((out[i].cpu().double() - ref).abs() <= bound).all(), i
 
 
+@pytest.mark.parametrize("T,heads", [(1, 1), (5, 8), (17, 9), (3, 128)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_mla_q_split(K, T, heads, interleaved):
+    """Heads in and out of whole groups, with the slab of nope dims and without; the record's latent dims are left alone."""
+    dev, g = _dev(), torch.Generator().manual_seed(T)
+    q = torch.randn(T, heads * 192, generator=g).to(torch.bfloat16).to(dev)
+    inv_freq = (10000.0 ** (-torch.arange(32) / 32.0)).to(dev)
+    positions = torch.randint(0, 100000, (T,), generator=g).to(dev, torch.int32)
+    qh = q.view(T, heads, 192).double()
+    ang = (positions.float()[:, None] * inv_freq)[:, None].double()
+    x0, x1 = (qh[..., 128::2], qh[..., 129::2]) if interleaved else (qh[..., 128:160], qh[..., 160:])
+    y0, y1 = x0 * ang.cos() - x1 * ang.sin(), x0 * ang.sin() + x1 * ang.cos()
+    ref = torch.stack((y0, y1), -1).flatten(-2) if interleaved else torch.cat((y0, y1), -1)
+    outs = []
+    for slab in (torch.full((heads, T + 3, 128), 7.0, dtype=torch.bfloat16, device=dev), None):
+        q_abs = torch.full((T, heads, 576), 5.0, dtype=torch.bfloat16, device=dev)
+        K.mla_q_split(q, inv_freq, positions, slab, q_abs, heads, interleaved)
+        torch.cuda.synchronize()
+        if slab is not None:
+            assert torch.equal(slab[:, :T], q.view(T, heads, 192)[..., :128].transpose(0, 1)) and (slab[:, T:] == 7.0).all()
+        assert (q_abs[..., :512] == 5.0).all()
+        # half an ulp of bf16; sine and cosine of the fp32 angle, two products and a sum: a few 2^-24 of |x0| + |x1|
+        bound = 2.0 ** -8 * ref.abs() + 2.0 ** -20 * 12
+        assert ((q_abs[..., 512:].double() - ref).abs() <= bound).all()
+        outs.append(q_abs)
+    assert torch.equal(*outs)
+
+
 def _mla_cfg():
     from cuteafd_b200.config import ModelConfig
     return ModelConfig(name="mla-moe-small", family="deepseek_v3", vocab_size=2048, num_layers=3, hidden=512,
