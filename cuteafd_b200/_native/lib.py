@@ -41,7 +41,8 @@ MAX_RANKS = 8
 WAIT_LIMIT_SETTERS = ("cafd_gemm_set_wait_limit_ns", "cafd_moe_set_wait_limit_ns", "cafd_attn_set_wait_limit_ns",
                       "cafd_gemm_fp8_set_wait_limit_ns", "cafd_tp_set_wait_limit_ns", "cafd_mla_set_wait_limit_ns",
                       "cafd_indexer_set_wait_limit_ns", "cafd_gemm_w4_set_wait_limit_ns", "cafd_gemm_exl3_set_wait_limit_ns",
-                      "cafd_decode_step_set_wait_limit_ns", "cafd_gemm_w8_set_wait_limit_ns", "cafd_attn_pair_set_wait_limit_ns")
+                      "cafd_decode_step_set_wait_limit_ns", "cafd_gemm_w8_set_wait_limit_ns", "cafd_attn_pair_set_wait_limit_ns",
+                      "cafd_gemm_split_set_wait_limit_ns")
 
 
 BOUNDS_UNITS = ("cafd_moe", "cafd_tp")        # translation units with checked peer-store sites

@@ -111,6 +111,7 @@ int cafd_argmax_candidates(const float* logits, float* cand_v, int* cand_i, int 
 int cafd_argmax_noalloc_max_rows(void);
 int cafd_argmax_noalloc(const float* logits, int* out, int T, int V, int ld, cafd_stream_t stream);
 int cafd_gemm_set_wait_limit_ns(unsigned long long ns);
+int cafd_gemm_split_set_wait_limit_ns(unsigned long long ns);
 
 // Block-scaled FP8 (E4M3) variant of cafd_gemm: same arguments plus w_scale / w_scale1 / x_scale.
 // K must be a multiple of 128; out is bf16.

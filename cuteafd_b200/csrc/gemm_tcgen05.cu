@@ -22,6 +22,8 @@ namespace cafd {
 
 bool skinny_takes(const cafd_gemm_args* a);                       // gemm_skinny.cu
 int skinny_dense(const cafd_gemm_args* a, cudaStream_t st);
+int gemm_split_parts(const cafd_gemm_args* a);                     // gemm_split.cu
+int gemm_split(const cafd_gemm_args* a, int splits, cudaStream_t st);
 
 constexpr int kBK = 64;            // K elements per stage (128 bytes of bf16: one swizzle atom)
 constexpr int kUmmaK = 16;         // K per tcgen05.mma for 16-bit inputs
@@ -591,6 +593,7 @@ extern "C" int cafd_gemm(const cafd_gemm_args* a, cafd_stream_t stream_) {
   if (a->rs_ranks < 0 || a->rs_ranks > 8 || a->n_signal_flags < 0 || a->n_signal_flags > 8 || (a->rs_ranks && a->rs_rows_per_rank <= 0)) return -16;
   if (a->wait_flag && !a->epoch) return -12;
   if (skinny_takes(a)) return skinny_dense(a, stream);
+  if (const int parts = gemm_split_parts(a)) return gemm_split(a, parts, stream);
   if (a->dual && a->glu) {
     if (!a->swap) return launch<false, true, 128, 128, true>(a, stream);
     switch (a->bx) {
