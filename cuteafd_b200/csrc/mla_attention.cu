@@ -99,8 +99,6 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* sC = smem + kQBytes;                 // two stages
   uint8_t* sP = smem + kQBytes + 2 * kKvBytes;
   uint8_t* sX = sP + kPBytes;
-  // the query atoms that go to TMEM arrive in the second stage, the probabilities' buffer and sX, all idle until then
-  auto staged = [&](int a) { return a < 4 ? sC + kKvBytes + a * (kMlaRows * 128) : a == 4 ? sP : sX; };
   auto s_max = reinterpret_cast<float (*)[2][kMlaRows]>(sX);       // [tile parity][half of the columns][row]; sums at the end
 
   // of a stage: k = the five atoms that only the scores read, v = the four that PV reads as well
@@ -156,6 +154,8 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tQ = tmem + kKvTile;          // + 32 * atom
   const uint32_t tO = tQ + kQTmem * 32;
 
+  // the query atoms that go to TMEM arrive in the second stage, the probabilities' buffer and sX, all idle until then
+  auto staged = [&](int a) { return a < 4 ? sC + kKvBytes + a * (kMlaRows * 128) : a == 4 ? sP : sX; };
   auto load_q = [&](int qrow) {
     mbar_expect_tx(&qt_in, kQTmem * kMlaRows * 128);
     for (int a = 0; a < kQTmem; ++a) tma_load_2d(staged(a), &tm_q, &qt_in, a * 64, qrow);

@@ -352,7 +352,7 @@ class GqaMoeEngine:
 
     def _exchange_launches(self, T: int) -> int:
         """Kernels one bf16 exchange launches for T tokens: plan (with the dispatch folded in for very small steps, three
-        launches wide from 8192 entries on), dispatch, fc1, fc2, combine."""
+        launches wide from ``WIDE_PLAN_ENTRIES`` entries on), dispatch, fc1, fc2, combine."""
         from ..parallel.moe_exchange import AttentionSide as A
         n = T * self.cfg.top_k
         fused = n <= A.FUSED_DISPATCH_ROWS and n * self.cfg.hidden * 2 <= A.FUSED_DISPATCH_BYTES
@@ -368,7 +368,9 @@ class GqaMoeEngine:
             K.linear(ws.ffn_d[:T], L.d_down, out=ws.h[:T], residual=ws.h[:T], resident=True)
             self.launches += 3
             return False
-        fused = T <= self.FUSED_ROUTE_TOKENS and cfg.hidden <= 8192 and hasattr(self.moe, "att")
+        # (the batch-invariant form keeps one route for every decode width)
+        most = self.FUSED_ROUTE_TOKENS if self.fixed_kv_split else min(self.FUSED_ROUTE_TOKENS, K.norm_route_rows(cfg.num_experts, cfg.hidden))
+        fused = T <= most and cfg.hidden <= 8192 and hasattr(self.moe, "att")
         logits = None
         if fused:
             K.norm_route(ws.h[:T], L.ln2, cfg.rms_eps, L.router, ws.x[:T], self.moe.att.idx[:T], self.moe.att.w[:T], cfg.top_k,
