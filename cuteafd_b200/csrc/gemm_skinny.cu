@@ -413,9 +413,9 @@ bool cafd::skinny_takes(const cafd_gemm_args* a) {
   const long long weights = static_cast<long long>(a->n_features) * a->k;        // of one of the two where there is a pair
   const bool rows = a->x_rows <= 8 ? (a->k <= 4096 ? weights <= (a->dual ? 50 : 200) * 1000000ll : tiles <= 2 * sms)
                                    : a->x_rows <= kSkMaxRows && a->k <= 4096 && tiles <= (a->x_rows <= 16 ? 4 : 1) * sms;
-  // tiles of 128 features whose K a cluster shares: 2048 x 4096 at 17 / 32 rows 13.1 / 17.1 us here, 6.7 / 7.6 there; 256 / 1024 x 7168 at
-  // 8 rows 10.0 / 10.7 and 4.2 / 5.8
-  if ((a->x_rows > 16 || (a->k > 4096 && tiles <= sms)) && gemm_split_parts(a)) return false;
+  // tiles of 128 features whose K a cluster shares: 2048 x 4096 at 9 / 17 / 32 rows 8.2 / 13.1 / 17.1 us here, 5.7 / 6.7 / 7.6 there, 256 /
+  // 1024 x 7168 at 8 rows 10.0 / 10.7 and 4.2 / 5.8 (but 128 x 2048 at 10 rows 3.3 here)
+  if ((a->x_rows > 16 || (a->k >= 4096 && tiles <= sms)) && gemm_split_parts(a)) return false;
   return a->swap && !a->fp8 && a->x_rows > 0 && rows && a->k % sk_elems(false) == 0 && !a->tile_expert && !a->row_dst &&
          !a->row_scale && !a->wait_flag && !a->signal_flag && !a->rs_ranks && !a->n_signal_flags && !(a->dual && a->glu) &&
          !(a->dual && (!a->w1 || a->w1_row_offset)) && fixed_kv_split_tokens() == 0 && aligned16(a->w0) && aligned16(a->w1) && aligned16(a->x);
